@@ -163,41 +163,35 @@ __device__ __forceinline__ void store_prim_cs(double2 *__restrict__ q, int c, co
 }
 
 // ------------------------------------------------------------------------------ fast reciprocals
-// FP64 path only (never FP64_EXACT): reciprocal and reciprocal square root from the single-
-// precision hardware approximations (PTX rcp.approx.ftz.f32 / rsqrt.approx.ftz.f32, relative error
-// below 2^-22), refined in one step by the truncated series of the exact correction.  With the seed
-// y0 and e = 1 - x y0 (|e| < 2^-22), 1/x = y0 / (1 - e) = y0 (1 + e + e^2 + ...); with
-// e = 1 - x y0^2, 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3e^2/8 + ...).  Keeping the terms up
-// to e^2 leaves a truncation error of order e^3 < 2^-66, far below double rounding: over 10^7 random
-// arguments and seed errors the results were within 1 (reciprocal) and 2 (reciprocal square root)
-// units in the last place of the correctly rounded values, where two Newton-Raphson steps (each
-// squares the error; Markstein, IBM J. Res. Dev. 34, 1990) gave up to 3, with a longer dependency
-// chain and more operations.  The seed is used when the single-precision argument lies in
-// [2^-99, 2^99) (its bits, sign included, between 0x0E000000 and 0x71000000: one integer compare
-// instead of two double-precision ones), so that seed and result are normal floats; anything else
-// (zero, tiny or huge magnitudes, negative arguments of the square root, NaN and Inf) takes the IEEE
-// double operation.
-__device__ __forceinline__ bool seed_ok(float xf) {
-    return __float_as_uint(xf) - 0x0E000000u < 0x63000000u;
+// FP64 path only (never FP64_EXACT): reciprocal and reciprocal square root from the hardware's coarse
+// double-precision approximations (PTX rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64: one instruction on the
+// argument's upper word, about 20 bits), refined in one step by the truncated series of the exact
+// correction.  With the seed y0 and e = 1 - x y0, 1/x = y0 / (1 - e) = y0 (1 + e + e^2 + ...); with
+// e = 1 - x y0^2, 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3e^2/8 + ...).  Keeping the terms up to
+// e^2 leaves a truncation error of order e^3, far below double rounding; y0 has at most 21 significant
+// bits, so y0^2 is exact.  The single-precision approximations give a seed of the same use but need the
+// argument converted to float and the seed back (two more instructions of the same slow pipe and their
+// latency on every face's dependency chain).  The seed is used for magnitudes in [2^-99, 2^99), tested
+// with one integer compare on the argument's upper word (sign included for the square root); anything
+// else (zero, tiny or huge magnitudes, negative arguments of the square root, NaN and Inf) takes the
+// IEEE double operation.
+__device__ __forceinline__ bool seed_ok(int hi) {
+    return (unsigned)hi - ((1023u - 99u) << 20) < (198u << 20);
 }
 
 __device__ __forceinline__ double rcp_nr(double x) {
-    const float xf = (float)x;
-    if (!seed_ok(fabsf(xf))) return 1.0 / x;
-    float yf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
-    const double y = (double)yf;
+    if (!seed_ok(__double2hiint(x) & 0x7fffffff)) return 1.0 / x;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);  // y (1 + e + e^2)
 }
 
 __device__ __forceinline__ double rsqrt_nr(double x) {
-    const float xf = (float)x;
-    if (!seed_ok(xf)) return rsqrt(x);
-    float yf;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
-    const double y = (double)yf;
-    const double e = fma(-(x * y), y, 1.0);
+    if (!seed_ok(__double2hiint(x))) return rsqrt(x);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);  // y (1 + e/2 + 3e^2/8)
 }
 
@@ -258,21 +252,26 @@ __device__ __forceinline__ void roe_exact(const Prim &L, const Prim &R, double n
 }
 
 // Fast: the same flux rearranged as F = (F_L + F_R - sum_k a_k r_k) / 2 with the wave strengths
-// a_k formed once, Roe weights from one reciprocal, c~ and 1/c~^2 from one rsqrt, and the left
-// sound speed from rsqrt(gamma p rho).  sl, sr = sqrt(rho) and rcl = rsqrt(gamma p_L rho_L) come
-// from the caller (the gather kernel computes them once per cell, the tile kernels once per face).
+// a_k formed once.  With r~ = sqrt(rho_L rho_R), the Roe weight sqrt(rho_L) / (sqrt(rho_L) +
+// sqrt(rho_R)) is rho_L / (rho_L + r~) and its complement r~ / (rho_L + r~): one root and one
+// reciprocal instead of two roots and one.  c~ and 1/c~^2 come from one rsqrt.  Harten's delta =
+// c_L / 15 needs a root only where the fix applies: |lambda| > delta is tested as 225 rho_L lambda^2 >
+// gamma p_L for the smaller |lambda| = ||V~| - c~|, and the fix is continuous at equality, so a
+// rounding-level difference there is one of the result too (a negative pressure takes the root, so
+// that it still ends in a NaN).
 // The FP64 kernels are compiled without multiply-add contraction and fuse where the source says
 // fma(), so the rounding is fixed by the source: every kernel variant, alone or batched, computes
 // the same bits whatever its register budget.
-__device__ __forceinline__ void roe_fast(const Prim &L, const Prim &R, double sl, double sr, double rcl,
-                                         double nx, double ny, double nz, double g, double F[5]) {
-    double inv = rcp_nr(sl + sr);
-    double wl = sl * inv, wr = sr * inv;
+__device__ __forceinline__ void roe_fast(const Prim &L, const Prim &R, double nx, double ny, double nz, double g,
+                                         double F[5]) {
+    const double rr = L.rho * R.rho;
+    const double rt = rr * rsqrt_nr(rr);
+    const double inv = rcp_nr(L.rho + rt);
+    double wl = L.rho * inv, wr = rt * inv;
     double ut = fma(L.u, wl, R.u * wr);
     double vt = fma(L.v, wl, R.v * wr);
     double wt = fma(L.w, wl, R.w * wr);
     double ht = fma(L.H, wl, R.H * wr);
-    double rt = sl * sr;
     double q2t = fma(ut, ut, fma(vt, vt, wt * wt));
     double c2 = (g - 1.0) * fma(-0.5, q2t, ht);
     double rc = rsqrt_nr(c2);
@@ -282,12 +281,12 @@ __device__ __forceinline__ void roe_fast(const Prim &L, const Prim &R, double sl
     double Vr = fma(R.u, nx, fma(R.v, ny, R.w * nz));
     double drho = R.rho - L.rho, dp = R.p - L.p, dV = Vr - Vl;
     double du = R.u - L.u, dv = R.v - L.v, dw = R.w - L.w;
-    // Harten's fix with delta = c_L / 15 (c_L = gamma p_L * rsqrt(gamma p_L rho_L))
-    double gpl = g * L.p;
-    double delta = (1.0 / 15.0) * (gpl * rcl);
     double lam1 = fabs(Vt - ct), lam5 = fabs(Vt + ct);
-    if (!(lam1 > delta) || !(lam5 > delta)) {
-        double h = 7.5 * (L.rho * rcl);  // 1 / (2 delta)
+    const double gpl = g * L.p, lmin = fabs(fabs(Vt) - ct);  // the smaller of the two
+    if (!(225.0 * L.rho * (lmin * lmin) > gpl) || __double2hiint(gpl) < 0) {
+        const double rcl = rsqrt_nr(gpl * L.rho);              // c_L = gamma p_L * rcl
+        const double delta = (1.0 / 15.0) * (gpl * rcl);
+        const double h = 7.5 * (L.rho * rcl);                  // 1 / (2 delta)
         if (!(lam1 > delta)) lam1 = fma(lam1, lam1, delta * delta) * h;
         if (!(lam5 > delta)) lam5 = fma(lam5, lam5, delta * delta) * h;
     }
@@ -366,6 +365,37 @@ __device__ __forceinline__ void ausm_fast(const Prim &L, const Prim &R, double r
     ausm_tail(L, R, cl, cr, Vl, Vr, Vl * (L.rho * rl), Vr * (R.rho * rr), nx, ny, nz, F);
 }
 
+// Fast: the flux through a symmetry face, between cell state d and its mirror image (the same density,
+// pressure and enthalpy, the normal velocity reversed).  The mirror symmetry leaves a normal force
+// only: mass, energy and tangential terms cancel.
+//   Roe: the averages are the cell's tangential flow, V~ = 0, c~^2 = (gamma - 1)(H - q_t^2 / 2) with
+//     q_t^2 the tangential speed squared, both acoustic waves move at c~ >= c (the entropy fix never
+//     applies), and the force is p + rho V (V + c~).
+//   AUSM: the split Mach numbers cancel and the two split pressures are equal, force 2 p P+(V / c).
+// About 30 operations for the general flux's 200, and no ghost enthalpy (two divisions): on the
+// 2-layer channels every cell has a symmetry face.
+__device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double ny, double nz, double g, int scheme,
+                                              double F[5]) {
+    const double V = fma(d.u, nx, fma(d.v, ny, d.w * nz));
+    double f;
+    if (scheme == 1) {
+        const double M = V * (d.rho * rsqrt_nr(g * d.p * d.rho));
+        double pp;
+        if (fabs(M) <= 1.0) pp = 0.25 * (M + 1.0) * (M + 1.0) * (2.0 - M);
+        else pp = M > 0.0 ? 1.0 : 0.0;
+        f = 2.0 * pp * d.p;
+    } else {
+        const double qt2 = fma(-V, V, fma(d.u, d.u, fma(d.v, d.v, d.w * d.w)));
+        const double c2 = (g - 1.0) * fma(-0.5, qt2, d.H);
+        f = fma(d.rho * V, V + c2 * rsqrt_nr(c2), d.p);
+    }
+    F[0] = 0.0;
+    F[1] = f * nx;
+    F[2] = f * ny;
+    F[3] = f * nz;
+    F[4] = 0.0;
+}
+
 // ------------------------------------------------------------------------------ ghost states
 // Ghost record: rho u v w p E H M.
 __device__ __forceinline__ void ghost_store(double *gp, double rho, double u, double v, double w, double p,
@@ -388,11 +418,17 @@ __device__ __forceinline__ void ghost_finish(double *gp, double g, double rho, d
     out = Prim{rho, u, v, w, p, H};
 }
 
+// Arithmetic of a stage kernel: the reference's own operations, restructured double precision, or
+// single-precision fluxes.
+enum : int { PREC_EXACT = 0, PREC_FAST = 1, PREC_F32 = 2 };
+
 // BC::Wall / BC::Symmetry (src/solver/PhysicalBC.cpp:124-231): mirrored velocity.  The kernels
 // never read a wall or symmetry ghost back (it is rebuilt from its interior cell at every stage), so
 // its record is written only when `store` says so (the last stage of an iteration, and
 // e3d_solver_residual): the state a run leaves is the same, with a fifth of the ghost writes.
-// Without the store only what the face flux needs is formed (H for symmetry faces).
+// Without the store only what the face flux needs is formed (H for symmetry faces; outside the exact
+// mode from one fast reciprocal instead of two divisions).
+template <int PREC>
 __device__ __forceinline__ void ghost_mirror(double *gp, double g, const Prim &d, double nx, double ny, double nz,
                                              Prim &out, bool store, bool need_h) {
     double V = d.u * nx + d.v * ny + d.w * nz;
@@ -406,8 +442,12 @@ __device__ __forceinline__ void ghost_mirror(double *gp, double g, const Prim &d
         double H = 0.0;
         if (need_h) {  // ghost_finish's E and H, in its operation order
             double q2 = u * u + v * v + w * w;
-            double E = d.p / ((g - 1) * d.rho) + (q2 / 2.0);
-            H = E + (d.p / d.rho);
+            if (PREC == PREC_EXACT) {
+                double E = d.p / ((g - 1) * d.rho) + (q2 / 2.0);
+                H = E + (d.p / d.rho);
+            } else {
+                H = fma(g, d.p * rcp_nr((g - 1.0) * d.rho), 0.5 * q2);  // gamma e + q^2 / 2
+            }
         }
         out = Prim{d.rho, u, v, w, d.p, H};
     }
@@ -480,23 +520,27 @@ __device__ __forceinline__ void block_sum_store(double v, double *dst) {
 // Boundary face of interior cell c (state me): updates its ghost cell (EulerSolver::updateBC,
 // src/solver/EulerSolver.cpp:201-251) and either writes the face flux to F (wall: pressure term,
 // :331-339; farfield / unclassified: physical flux of the ghost, :349-357) and returns false, or
-// leaves the mirrored ghost in gs and returns true (symmetry: Roe against the ghost, :343-346).
+// leaves the mirrored ghost in gs and returns true (symmetry: Roe against the ghost, :343-346).  The
+// FP64 mode forms the symmetry flux here too and always returns false.
+template <int PREC>
 __device__ __forceinline__ bool boundary_face(const StageArgs &a, int tag, double *gp, int c, const Prim &me,
                                               const double4 &fg, double F[5], Prim &gs) {
     const double g = a.gamma;
     const bool store = a.last_stage || a.residual_only || a.ghost_out;
     if (tag == TAG_WALL) {
-        ghost_mirror(gp, g, me, fg.x, fg.y, fg.z, gs, store, false);
+        ghost_mirror<PREC>(gp, g, me, fg.x, fg.y, fg.z, gs, store, false);
         F[0] = 0;
-        F[1] = fg.x * gs.p;
-        F[2] = fg.y * gs.p;
-        F[3] = fg.z * gs.p;
+        F[1] = fg.x * me.p;
+        F[2] = fg.y * me.p;
+        F[3] = fg.z * me.p;
         F[4] = 0;
         return false;
     }
     if (tag == TAG_SYM) {
-        ghost_mirror(gp, g, me, fg.x, fg.y, fg.z, gs, store, true);
-        return true;
+        ghost_mirror<PREC>(gp, g, me, fg.x, fg.y, fg.z, gs, store, PREC != PREC_FAST);
+        if (PREC != PREC_FAST) return true;
+        sym_flux_fast(me, fg.x, fg.y, fg.z, g, a.scheme, F);
+        return false;
     }
     if (tag == TAG_FAR) {
         double q2 = me.u * me.u + me.v * me.v + me.w * me.w;
@@ -623,12 +667,8 @@ __global__ void __launch_bounds__(kStageThreads, MINB) stage_kernel(StageArgs a)
     double r2 = 0.0;
     if (c < a.n_cells) {
         const Prim me = load_prim(a.qin, c);
-        // sqrt(rho) and rsqrt(gamma p rho) of this cell, shared by all its faces (fast path)
-        double s_me = 0.0, r_me = 0.0;
-        if (!EXACT) {
-            s_me = me.rho * rsqrt_nr(me.rho);
-            r_me = rsqrt_nr(g * me.p * me.rho);
-        }
+        // rsqrt(gamma p rho) of this cell, for the time step and AUSM's sound speed (fast path)
+        const double r_me = EXACT ? 0.0 : rsqrt_nr(g * me.p * me.rho);
         double R[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         const int e0 = a.cptr[c], e1 = a.cptr[c + 1];
         for (int e = e0; e < e1; e++) {
@@ -643,33 +683,31 @@ __global__ void __launch_bounds__(kStageThreads, MINB) stage_kernel(StageArgs a)
             Prim fl, fr;
             double sS = fg.w;
             bool roe = true;
-            double s_l = s_me, s_r = s_me, r_l = r_me, r_nb = r_me;
+            double r_l = r_me, r_r = r_me;
             if (tag <= TAG_RIGHT) {
                 const Prim nb = load_prim(a.qin, idx);
                 const bool left = tag == TAG_LEFT;
                 fl = left ? me : nb;
                 fr = left ? nb : me;
                 sS = left ? fg.w : -fg.w;
-                if (!EXACT) {
-                    double s_nb = nb.rho * rsqrt_nr(nb.rho);
-                    r_nb = rsqrt_nr(g * nb.p * nb.rho);
-                    s_l = left ? s_me : s_nb;
-                    s_r = left ? s_nb : s_me;
+                if (!EXACT && a.scheme == 1) {
+                    const double r_nb = rsqrt_nr(g * nb.p * nb.rho);
                     r_l = left ? r_me : r_nb;
+                    r_r = left ? r_nb : r_me;
                 }
             } else {
                 Prim gs;
-                roe = boundary_face(a, tag, a.ghost + 8 * (size_t)idx, c, me, fg, F, gs);
+                roe = boundary_face<EXACT ? PREC_EXACT : PREC_FAST>(a, tag, a.ghost + 8 * (size_t)idx, c, me, fg, F, gs);
                 fl = me;
-                fr = gs;  // symmetry ghost: rho and p are the cell's, so s_r = s_me
+                fr = gs;  // symmetry ghost
             }
             if (roe) {
                 if (a.scheme == 1) {
                     if (EXACT) ausm_exact(fl, fr, fg.x, fg.y, fg.z, g, F);
-                    else ausm_fast(fl, fr, r_l, tag == TAG_LEFT ? r_nb : r_me, fg.x, fg.y, fg.z, g, F);
+                    else ausm_fast(fl, fr, r_l, r_r, fg.x, fg.y, fg.z, g, F);
                 } else {
                     if (EXACT) roe_exact(fl, fr, fg.x, fg.y, fg.z, g, F);
-                    else roe_fast(fl, fr, s_l, s_r, r_l, fg.x, fg.y, fg.z, g, F);
+                    else roe_fast(fl, fr, fg.x, fg.y, fg.z, g, F);
                 }
             }
 #pragma unroll
@@ -739,22 +777,13 @@ __global__ void __launch_bounds__(NT) colour_kernel(StageArgs a, const ColourFac
         if (a.scheme == 1)
             ausm_fast(L, R, rsqrt_nr(g * L.p * L.rho), rsqrt_nr(g * R.p * R.rho), fg.x, fg.y, fg.z, g, F);
         else
-            roe_fast(L, R, L.rho * rsqrt_nr(L.rho), R.rho * rsqrt_nr(R.rho), rsqrt_nr(g * L.p * L.rho), fg.x, fg.y,
-                     fg.z, g, F);
+            roe_fast(L, R, fg.x, fg.y, fg.z, g, F);
         colour_add(rc, cf.l, F, fg.w, true);
         colour_add(rc, cf.r, F, fg.w, false);
         return;
     }
     Prim gs;
-    if (boundary_face(a, cf.tag, a.ghost + 8 * (size_t)cf.r, cf.l, L, fg, F, gs)) {
-        // symmetry ghost: rho and p are the cell's
-        const double rl = rsqrt_nr(g * L.p * L.rho);
-        if (a.scheme == 1) ausm_fast(L, gs, rl, rl, fg.x, fg.y, fg.z, g, F);
-        else {
-            const double sl = L.rho * rsqrt_nr(L.rho);
-            roe_fast(L, gs, sl, sl, rl, fg.x, fg.y, fg.z, g, F);
-        }
-    }
+    boundary_face<PREC_FAST>(a, cf.tag, a.ghost + 8 * (size_t)cf.r, cf.l, L, fg, F, gs);
     colour_add(rc, cf.l, F, fg.w, true);
 }
 
@@ -847,7 +876,7 @@ constexpr int kWaitLimit = 1 << 22;  // polls of a barrier before the kernel giv
 __device__ __forceinline__ uint32_t round16(uint32_t b) { return (b + 15u) & ~15u; }
 
 // ------------------------------------------------------------------------------ face tiles
-// A tile is kTileCells consecutive cells (a spatially compact group in the Morton cell order).
+// A tile is kTileCells consecutive cells (a spatially compact group in the spatial cell order).
 // Its data, staged in shared memory:
 //   st[LC]   48-byte states: owned cells (one bulk copy) then halo cells (outside neighbours,
 //            gathered with cp.async)
@@ -914,10 +943,9 @@ __device__ __forceinline__ Prim tile_prim(const double2 *st, int i) {
     return Prim{x.x, x.y, y.x, y.y, z.x, z.y};
 }
 
-// One flux per tile face; F*S of face j replaces record j (fs[5 j + k] aliases b.rec[j]).  The fast
-// path takes sqrt(rho) and rsqrt(gamma p rho) of both sides per face: a per-cell pass over the tile
-// before the fluxes would cost a barrier phase and 16 bytes of shared memory per local cell, and
-// measured slower on B200.
+// One flux per tile face; F*S of face j replaces record j (fs[5 j + k] aliases b.rec[j]).  Roots of
+// the face's states are taken per face: a per-cell pass over the tile before the fluxes would cost a
+// barrier phase and 16 bytes of shared memory per local cell, and measured slower on B200.
 template <bool EXACT, int NT>
 __device__ __forceinline__ void tile_fluxes(const StageArgs &a, const TileBuf &b, double *fs, int nf, int c0,
                                             int tid) {
@@ -937,34 +965,25 @@ __device__ __forceinline__ void tile_fluxes(const StageArgs &a, const TileBuf &b
                 else ausm_fast(L, R, rsqrt_nr(g * L.p * L.rho), rsqrt_nr(g * R.p * R.rho), fg.x, fg.y, fg.z, g, F);
             } else {
                 if (EXACT) roe_exact(L, R, fg.x, fg.y, fg.z, g, F);
-                else
-                    roe_fast(L, R, L.rho * rsqrt_nr(L.rho), R.rho * rsqrt_nr(R.rho), rsqrt_nr(g * L.p * L.rho), fg.x,
-                             fg.y, fg.z, g, F);
+                else roe_fast(L, R, fg.x, fg.y, fg.z, g, F);
             }
         } else {
             Prim gs;
             double *gp = a.ghost + 8 * (size_t)fr.ghost;
-            if (boundary_face(a, tag, gp, c0 + l, L, fg, F, gs)) {
-                // the ghost's density and pressure are the interior cell's (mirror)
-                if (a.scheme == 1) {
-                    if (EXACT) ausm_exact(L, gs, fg.x, fg.y, fg.z, g, F);
-                    else {
-                        const double rl = rsqrt_nr(g * L.p * L.rho);
-                        ausm_fast(L, gs, rl, rl, fg.x, fg.y, fg.z, g, F);
-                    }
-                } else {
-                    if (EXACT) roe_exact(L, gs, fg.x, fg.y, fg.z, g, F);
-                    else {
-                        const double sl = L.rho * rsqrt_nr(L.rho);
-                        roe_fast(L, gs, sl, sl, rsqrt_nr(g * L.p * L.rho), fg.x, fg.y, fg.z, g, F);
-                    }
-                }
+            if (boundary_face<EXACT ? PREC_EXACT : PREC_FAST>(a, tag, gp, c0 + l, L, fg, F, gs)) {
+                // exact mode's symmetry face: the general flux against the mirrored ghost
+                if (a.scheme == 1) ausm_exact(L, gs, fg.x, fg.y, fg.z, g, F);
+                else roe_exact(L, gs, fg.x, fg.y, fg.z, g, F);
             }
         }
-        // the record is in registers; keep the compiler from moving its loads past the overwrite
+        // The area is read again here instead of held through the flux (two registers that would spill
+        // at seven blocks per SM); the fences keep the compiler from merging the two reads and from
+        // moving a read of the record past the overwrite.
+        asm volatile("" ::: "memory");
+        const double S = b.rec[j].S;
         asm volatile("" ::: "memory");
 #pragma unroll
-        for (int k = 0; k < 5; k++) fs[5 * j + k] = F[k] * fg.w;
+        for (int k = 0; k < 5; k++) fs[5 * j + k] = F[k] * S;
     }
 }
 

@@ -1,7 +1,7 @@
 // FP32_FLUX stage kernel: fluxes, face states and the time step in single precision; the
 // conservative state W0, the residual sums, the Runge-Kutta update and every reduction in double.
 //
-// Same face-tile scheme as tile_kernel (stage.cuh): one block per tile of kTileCells Morton-ordered
+// Same face-tile scheme as tile_kernel (stage.cuh): one block per tile of kTileCells consecutive
 // cells, bulk copies of the tile's contiguous data plus cp.async gathers of its halo onto one
 // mbarrier, each face evaluated once, each cell summing its faces' F*S in ascending reference face
 // id (deterministic).  Cell records are 32 bytes (two float4), face records 24 bytes, so a tile's
@@ -159,7 +159,7 @@ __device__ __forceinline__ void tile_fluxes_f32(const StageArgs &a, const Tile32
             const double4 fg = make_double4(fr.nx, fr.ny, fr.nz, fr.S);
             double Fd[5];
             Prim gs;
-            if (boundary_face(a, tag, a.ghost + 8 * (size_t)fr.ghost, c0 + l, Ld, fg, Fd, gs)) {
+            if (boundary_face<PREC_F32>(a, tag, a.ghost + 8 * (size_t)fr.ghost, c0 + l, Ld, fg, Fd, gs)) {
                 const PrimF G{(float)gs.rho, (float)gs.u, (float)gs.v, (float)gs.w, (float)gs.p, (float)gs.H, L.s, L.r};
                 if (a.scheme == 1) ausm_f32(L, G, fr.nx, fr.ny, fr.nz, gf, F);
                 else roe_f32(L, G, fr.nx, fr.ny, fr.nz, gf, F);
