@@ -4,7 +4,7 @@
 Workload (default): the large all-tetrahedral roofline mesh -- a 128^3 hexahedral box [0,4]^3
 with a Gaussian floor bump (height 0.1, sigma 0.3), every hexahedron split into 6 tetrahedra
 (12,582,912 cells, 25,264,128 faces), nodes jittered 3% (seed 2), Mach 0.6, AoA 0, Roe, CFL 1.0,
-FP64, Morton (spatial) cell order on the device.  Synthetic, generated in-process (no dataset).
+FP64, spatial (compact groups) cell order on the device.  Synthetic, generated in-process (no dataset).
 
 A step is one RK5 iteration (5 stages over every cell, with ghost updates, local time step,
 update, density-RMS reduction and force sampling).  ``value`` counts 5 x cells x steps per

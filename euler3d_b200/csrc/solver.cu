@@ -17,6 +17,7 @@
 #include "euler3d_b200.h"
 #include "solver.hpp"
 #include "stage_ws.cuh"
+#include "tile_order.hpp"
 
 namespace e3d {
 
@@ -760,40 +761,22 @@ static void build_tiles(Solver *S, const std::vector<int> &cptr, const std::vect
     S->tile_faces_total = (int64_t)tface.size();
 }
 
-// Morton order of approximate cell centres (mean of the cell's face centres): consecutive cells
-// form spatially compact groups, which keeps the halo of a face tile small.
+// Compact tiles (tile_order.hpp) of the cells by approximate cell centres (mean of the cell's face
+// centres).
 static std::vector<int> spatial_order(const e3d_mesh_desc *d) {
     const int N = d->n_cells;
     std::vector<double> cx(3 * (size_t)N);
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     for (int c = 0; c < N; c++) {
         double s[3] = {0, 0, 0};
         int n = d->cell2face_ptr[c + 1] - d->cell2face_ptr[c];
         for (int k = d->cell2face_ptr[c]; k < d->cell2face_ptr[c + 1]; k++)
             for (int q = 0; q < 3; q++) s[q] += d->face_center[3 * (size_t)d->cell2face[k] + q];
         for (int q = 0; q < 3; q++) {
-            cx[3 * (size_t)c + q] = s[q] / std::max(n, 1);
-            lo[q] = std::min(lo[q], cx[3 * (size_t)c + q]);
-            hi[q] = std::max(hi[q], cx[3 * (size_t)c + q]);
+            const double x = s[q] / std::max(n, 1);
+            cx[3 * (size_t)c + q] = std::fabs(x) < 1e100 ? x : 0.0;  // any number orders; NaN would not
         }
     }
-    double ext = std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1e-300});
-    std::vector<std::pair<uint64_t, int>> key(N);
-    for (int c = 0; c < N; c++) {
-        uint64_t qv[3];
-        for (int q = 0; q < 3; q++) {
-            double u = (cx[3 * (size_t)c + q] - lo[q]) / ext;
-            qv[q] = (uint64_t)std::min(std::max(u, 0.0) * 2097151.0, 2097151.0);
-        }
-        uint64_t m = 0;
-        for (int b = 0; b < 21; b++)
-            for (int q = 0; q < 3; q++) m |= ((qv[q] >> b) & 1ull) << (3 * b + q);
-        key[c] = {m, c};
-    }
-    std::sort(key.begin(), key.end());
-    std::vector<int> order(N);
-    for (int c = 0; c < N; c++) order[c] = key[c].second;
-    return order;
+    return compact_tile_order(N, d->n_faces_int, d->face2cell, d->face_unit_normal, cx, kTileCells);
 }
 
 static void create_solver(const e3d_mesh_desc *d, const e3d_flow_params *p, Solver *S) {

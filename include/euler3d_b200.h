@@ -52,8 +52,8 @@ enum { E3D_SCHEME_ROE = 0, E3D_SCHEME_AUSM = 1 };
 enum { E3D_PREC_FP64_EXACT = 0, E3D_PREC_FP64 = 1, E3D_PREC_FP32_FLUX = 2 };
 
 /* Cell ordering used on the device (results are always returned in reference order):
- * reference order, reverse Cuthill-McKee of the cell graph, or Morton order of the cell centres
- * (spatially compact groups of cells, which the face-tile kernel needs). */
+ * reference order, reverse Cuthill-McKee of the cell graph, or recursive bisection into spatially
+ * compact groups of cells (which the face-tile kernels need). */
 enum { E3D_ORDER_NATIVE = 0, E3D_ORDER_RCM = 1, E3D_ORDER_SPATIAL = 2 };
 
 /* Time integration (the reference's TIME_INTEGRATION= key, src/parser/SimConfig.cpp:130-148, and
