@@ -30,6 +30,9 @@ SOURCES = [
     ("stage_exact.cu", ["-fmad=false"]),
     ("stage_fast.cu", ["-fmad=false"]),
     ("stage_f32.cu", ["-fmad=false"]),
+    ("resident_exact.cu", ["-fmad=false"]),
+    ("resident_fast.cu", ["-fmad=false"]),
+    ("resident_f32.cu", ["-fmad=false"]),
     ("solver.cu", ["-fmad=false"]),
     ("batch.cu", ["-fmad=false"]),
     ("outputs.cu", ["-fmad=false"]),

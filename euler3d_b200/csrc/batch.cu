@@ -221,7 +221,7 @@ struct Batch {
                 bs.parity = p ^ (s & 1);
                 launch_stage(bs);
             }
-            launch_finalize_batch(fargs.p, counts.p + 1, member_cap, stream);
+            launch_finalize_batch(fargs.p, counts.p + 1, member_cap, precision == E3D_PREC_FP64_EXACT, stream);
             launch_coeff_batch(cargs.p, counts.p + 1, 1 - p, member_cap, stream);
         }
         launch_control_gather(ctlp.p, counts.p + 1, ctl_all.p, member_cap, stream);

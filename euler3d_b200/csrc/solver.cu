@@ -23,231 +23,34 @@ namespace e3d {
 
 
 // ------------------------------------------------------------------------------ small kernels
-
-// Sum of the per-block partials in a fixed order, RMS, and the stop tests of
-// EulerSolver::Run (src/solver/EulerSolver.cpp:96-112).  One block per solver; `sh` is the block's
-// kReduceThreads-entry scratch.
-__device__ __forceinline__ void finalize_body(const FinalizeArgs &f, double *sh) {
-    Control *ctl = f.ctl;
-    if (ctl->done) return;
-    if (ctl->fault) {  // a stage kernel's bounded wait gave up: its cells kept their old state, so stop
-        if (threadIdx.x == 0) {
-            ctl->done = 1;
-            ctl->stop_reason = E3D_STOP_MAX_ITER;
-        }
-        return;
-    }
-    if (f.rsq) {
-        // FP64_EXACT: EulerSolver::computeRMS's own order, one running sum over the cells in
-        // reference order (src/solver/EulerSolver.cpp:382-389)
-        if (threadIdx.x != 0) return;
-        double s = 0.0;
-        for (int i = 0; i < f.n_cells; i++) s += f.rsq[i];
-        sh[0] = s;
-    } else {
-        double v = 0.0;
-        for (int i = threadIdx.x; i < f.n_part; i += kReduceThreads) v += f.partials[i];
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int s = kReduceThreads / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-            __syncthreads();
-        }
-        if (threadIdx.x != 0) return;
-    }
-    double rms = sqrt(sh[0] / f.n_domain);
-    if (ctl->n_rms < ctl->hist_cap) f.hist[ctl->n_rms] = rms;
-    if (ctl->n_rms == 0) ctl->rms0 = rms;
-    ctl->n_rms += 1;
-    ctl->last_rms = rms;
-    ctl->minit_valid = 0;
-    ctl->sample_now = 0;
-    if (!isfinite(rms)) {  // the reference would spin to MAX_ITER on a NaN; stop and report it
-        ctl->nonfinite = 1;
-        ctl->done = 1;
-        ctl->stop_reason = E3D_STOP_MAX_ITER;
-        return;
-    }
-    if (rms < ctl->min_res || (ctl->min_drop > 0.0 && rms < ctl->min_drop * ctl->rms0)) {
-        ctl->done = 1;
-        ctl->stop_reason = E3D_STOP_RESIDUAL;
-        return;
-    }
-    if (ctl->stall_window > 0 && (ctl->stall_below <= 0.0 || rms < ctl->stall_below * ctl->rms0)) {
-        // the residual has stopped falling (a precision floor)
-        if (ctl->best_rms == 0.0 || rms < ctl->best_rms) {
-            ctl->best_rms = rms;
-            ctl->since_best = 0;
-        } else if (++ctl->since_best >= ctl->stall_window) {
-            ctl->done = 1;
-            ctl->stop_reason = E3D_STOP_STALL;
-            return;
-        }
-    }
-    ctl->it += 1;
-    if (ctl->it % ctl->sampling == 0) {
-        ctl->sample_now = 1;
-    } else if (ctl->it >= ctl->max_iter) {
-        ctl->done = 1;
-        ctl->stop_reason = E3D_STOP_MAX_ITER;
-    }
-}
-
-__global__ void __launch_bounds__(kReduceThreads) finalize_kernel(FinalizeArgs f) {
-    __shared__ double sh[kReduceThreads];
-    finalize_body(f, sh);
+template <int NT>
+__global__ void __launch_bounds__(NT) finalize_kernel(FinalizeArgs f) {
+    __shared__ ControlScratch sh;
+    finalize_body<NT>(f, f.ctl, f.partials, sh);
 }
 
 // Block m: member m of a batch.
-__global__ void __launch_bounds__(kReduceThreads) finalize_batch_kernel(const FinalizeArgs *__restrict__ f,
-                                                                        const int *__restrict__ n_members) {
+template <int NT>
+__global__ void __launch_bounds__(NT) finalize_batch_kernel(const FinalizeArgs *__restrict__ f,
+                                                            const int *__restrict__ n_members) {
     if ((int)blockIdx.x >= *n_members) return;
-    __shared__ double sh[kReduceThreads];
+    __shared__ ControlScratch sh;
     const FinalizeArgs a = f[blockIdx.x];
-    finalize_body(a, sh);
-}
-
-__device__ __forceinline__ double wall_pressure(const CoeffArgs &a, int c) {
-    if (!a.w0) return a.q[3 * c + 2].x;
-    const size_t st = (size_t)a.w0_stride;
-    const double rho = a.w0[c], mu = a.w0[st + c], mv = a.w0[2 * st + c], mw = a.w0[3 * st + c];
-    return (a.gamma - 1.0) * (a.w0[4 * st + c] - 0.5 * (mu * mu + mv * mv + mw * mw) / rho);
-}
-
-// AeroCoefficients::Update (src/solver/AeroCoefficients.cpp:38-52): face terms in parallel, summed
-// by one thread in the reference's wall order so the sums are the reference's; then
-// EulerSolver::ConvergenceCriteria and the CL/CD/CM selection (src/solver/EulerSolver.cpp:132-152, :253-279).
-// One block per solver; `terms` is the block's 6 x kCoeffThreads scratch.
-__device__ __forceinline__ void coeff_body(const CoeffArgs &a, double (*terms)[kCoeffThreads]) {
-    Control *ctl = a.ctl;
-    if (a.run_mode && (ctl->done || !ctl->sample_now)) return;
-    double F[3] = {0, 0, 0}, CP[3] = {0, 0, 0};
-    if (a.sequential) {
-        // the reference's order: one running sum over the wall list
-        for (int base = 0; base < a.n_wall; base += kCoeffThreads) {
-            int i = base + threadIdx.x;
-            if (i < a.n_wall) {
-                double p = wall_pressure(a, a.cell[i]);
-                double cp = a.cp_factor * (p - a.p_inf);
-                if (a.cp_out) a.cp_out[i] = cp;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    double coeff = a.svec[3 * i + k] * cp * a.cref / a.sref;
-                    terms[k][threadIdx.x] = coeff;
-                    terms[3 + k][threadIdx.x] = coeff * a.center[3 * i + k];
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int n = min(kCoeffThreads, a.n_wall - base);
-                for (int j = 0; j < n; j++) {
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        F[k] += terms[k][j];
-                        CP[k] += terms[3 + k][j];
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    } else {
-        // fixed-shape tree: strided per-thread sums over wall faces t, t + T, t + 2T, ... in that
-        // order (their loads issued four faces at a time), then a pairwise tree (deterministic)
-        constexpr int U = 4;
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        for (int base = threadIdx.x; base < a.n_wall; base += U * kCoeffThreads) {
-            double p[U], sv[U][3], ce[U][3];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int i = base + u * kCoeffThreads;
-                if (i < a.n_wall) {
-                    p[u] = wall_pressure(a, a.cell[i]);
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        sv[u][k] = a.svec[3 * i + k];
-                        ce[u][k] = a.center[3 * i + k];
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                if (base + u * kCoeffThreads >= a.n_wall) break;
-                const double cp = a.cp_factor * (p[u] - a.p_inf);
-                if (a.cp_out) a.cp_out[base + u * kCoeffThreads] = cp;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const double coeff = sv[u][k] * cp * a.cref / a.sref;
-                    acc[k] += coeff;
-                    acc[3 + k] += coeff * ce[u][k];
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 6; k++) terms[k][threadIdx.x] = acc[k];
-        __syncthreads();
-        for (int st = kCoeffThreads / 2; st > 0; st >>= 1) {
-            if (threadIdx.x < st)
-#pragma unroll
-                for (int k = 0; k < 6; k++) terms[k][threadIdx.x] += terms[k][threadIdx.x + st];
-            __syncthreads();
-        }
-        for (int k = 0; k < 3; k++) {
-            F[k] = terms[k][0];
-            CP[k] = terms[3 + k][0];
-        }
-    }
-    if (threadIdx.x != 0) return;
-    double lever[3] = {a.ref[0] - CP[0], a.ref[1] - CP[1], a.ref[2] - CP[2]};
-    double M[3] = {(F[1] * lever[2] - F[2] * lever[1]) / a.cref, (F[2] * lever[0] - F[0] * lever[2]) / a.cref,
-                   (F[0] * lever[1] - F[1] * lever[0]) / a.cref};
-    if (!a.run_mode) {
-        for (int k = 0; k < 3; k++) {
-            a.out[k] = F[k];
-            a.out[3 + k] = M[k];
-        }
-        return;
-    }
-    double cl = F[a.axis[0]] * a.sign[0], cd = F[a.axis[1]] * a.sign[1], cm = M[a.axis[2]] * a.sign[2];
-    double tol = ctl->min_aero;
-    bool ok = fabs(ctl->cl - cl) < tol && fabs(ctl->cd - cd) < tol && fabs(ctl->cm - cm) < tol;
-    ctl->counter = ok ? ctl->counter + 1 : 0;
-    if (a.samples && ctl->n_samples < ctl->sample_cap) {  // a residuals.dat row (EulerSolver::PrintInfo)
-        double *s = a.samples + 7 * (size_t)ctl->n_samples;
-        s[0] = ctl->it;
-        for (int k = 0; k < 3; k++) {
-            s[1 + k] = F[k];
-            s[4 + k] = M[k];
-        }
-    }
-    ctl->n_samples += 1;
-    ctl->cl = cl;
-    ctl->cd = cd;
-    ctl->cm = cm;
-    for (int k = 0; k < 3; k++) {
-        ctl->force[k] = F[k];
-        ctl->moment[k] = M[k];
-    }
-    if (ctl->counter >= 2) {
-        ctl->done = 1;
-        ctl->stop_reason = E3D_STOP_COEFFICIENTS;
-    } else if (ctl->it >= ctl->max_iter) {
-        ctl->done = 1;
-        ctl->stop_reason = E3D_STOP_MAX_ITER;
-    }
+    finalize_body<NT>(a, a.ctl, a.partials, sh);
 }
 
 __global__ void __launch_bounds__(kCoeffThreads) coeff_kernel(CoeffArgs a) {
-    __shared__ double terms[6][kCoeffThreads];
-    coeff_body(a, terms);
+    __shared__ ControlScratch sh;
+    coeff_body<kCoeffThreads>(a, a.ctl, sh);
 }
 
 // Block m: member m of a batch, its arguments for the state buffer `parity`.
 __global__ void __launch_bounds__(kCoeffThreads) coeff_batch_kernel(const CoeffArgs *__restrict__ c,
                                                                     const int *__restrict__ n_members, int parity) {
     if ((int)blockIdx.x >= *n_members) return;
-    __shared__ double terms[6][kCoeffThreads];
+    __shared__ ControlScratch sh;
     const CoeffArgs a = c[2 * blockIdx.x + parity];
-    coeff_body(a, terms);
+    coeff_body<kCoeffThreads>(a, a.ctl, sh);
 }
 
 // Control blocks of a batch's members into one array (read back with one copy).
@@ -325,10 +128,15 @@ void launch_smooth(const SmoothArgs &a, cudaStream_t s) {
     smooth_kernel<<<(a.n_cells + kSmoothThreads - 1) / kSmoothThreads, kSmoothThreads, 0, s>>>(a);
 }
 
-void launch_finalize(const FinalizeArgs &f, cudaStream_t s) { finalize_kernel<<<1, kReduceThreads, 0, s>>>(f); }
+// FP64_EXACT's sum over every cell takes a larger block than the sum of the block partials.
+void launch_finalize(const FinalizeArgs &f, cudaStream_t s) {
+    if (f.rsq) finalize_kernel<kOrderedThreads><<<1, kOrderedThreads, 0, s>>>(f);
+    else finalize_kernel<kReduceThreads><<<1, kReduceThreads, 0, s>>>(f);
+}
 void launch_coeff(const CoeffArgs &c, cudaStream_t s) { coeff_kernel<<<1, kCoeffThreads, 0, s>>>(c); }
-void launch_finalize_batch(const FinalizeArgs *f, const int *n_members, int grid, cudaStream_t s) {
-    finalize_batch_kernel<<<grid, kReduceThreads, 0, s>>>(f, n_members);
+void launch_finalize_batch(const FinalizeArgs *f, const int *n_members, int grid, bool exact, cudaStream_t s) {
+    if (exact) finalize_batch_kernel<kOrderedThreads><<<grid, kOrderedThreads, 0, s>>>(f, n_members);
+    else finalize_batch_kernel<kReduceThreads><<<grid, kReduceThreads, 0, s>>>(f, n_members);
 }
 void launch_coeff_batch(const CoeffArgs *c, const int *n_members, int parity, int grid, cudaStream_t s) {
     coeff_batch_kernel<<<grid, kCoeffThreads, 0, s>>>(c, n_members, parity);
@@ -679,15 +487,24 @@ static void build_tiles(Solver *S, const std::vector<int> &cptr, const std::vect
             face_local[inter_slot[i]] = (int)tface.size() - fbase;
             tface.push_back(inter[i]);
         }
-        std::vector<int> bnd_local(bnd.size());
-        for (size_t b = 0; b < bnd.size(); b++) {
+        // boundary faces by kind (farfield and unclassified ones first, where the resident kernel
+        // expects them): a warp's faces mostly take one branch
+        std::vector<int> bnd_local(bnd.size()), by_kind(bnd.size());
+        std::iota(by_kind.begin(), by_kind.end(), 0);
+        std::stable_sort(by_kind.begin(), by_kind.end(), [&](int x, int y) {
+            return (cf[bnd[x]].x & ((1 << kTagBits) - 1)) > (cf[bnd[y]].x & ((1 << kTagBits) - 1));
+        });
+        int n_far = 0;
+        for (int b : by_kind) {
             int e = bnd[b];
             int tag = cf[e].x & ((1 << kTagBits) - 1);
+            n_far += tag >= TAG_FAR;
             int c = (int)(std::upper_bound(cptr.begin(), cptr.end(), e) - cptr.begin()) - 1;
             bnd_local[b] = (int)tface.size() - fbase;
             const double4 gq = fgeo[cf[e].y];
             tface.push_back(FaceRec{local(c) | (tag << (2 * kTileLocalBits)), cf[e].y - Fint, gq.x, gq.y, gq.z, gq.w});
         }
+        S->max_far = std::max(S->max_far, n_far);
         const int nfaces = (int)tface.size() - fbase;
         if (nfaces >= (1 << 15)) {
             ok = false;
@@ -1035,6 +852,7 @@ static void create_solver(const e3d_mesh_desc *d, const e3d_flow_params *p, Solv
     E3D_CUDA(cudaMemsetAsync(S->ctl, 0, sizeof(Control), s));
     E3D_CUDA(cudaEventCreate(&S->ev0));
     E3D_CUDA(cudaEventCreate(&S->ev1));
+    S->plan_resident();
     S->new2old = std::move(new2old);
     S->ghost_ref = std::move(ghost_ref);
     E3D_CUDA(cudaStreamSynchronize(s));
@@ -1335,12 +1153,36 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
                 S->graph = nullptr;
             }
             S->variant = v;
+            S->variant_forced = true;
         }
         int64_t launches = 0;
         double stage_ms = 0.0;
         int64_t stage_launches = 0;
         if (rp->profile_stages < 0 || rp->profile_stages > 2) throw Error(E3D_ERR_INVALID_ARG, "profile_stages must be 0, 1 or 2");
-        if (rp->profile_stages != 1) {
+        // Blocks that wait for one another need the whole grid on the GPU: one resident run per device
+        // at a time in this process (a run beside it takes the stage kernels, with the same results).
+        static std::mutex resident_busy[64];
+        std::unique_lock<std::mutex> resident;
+        if (rp->profile_stages == 0 && !S->variant_forced && S->device < 64 && S->resident_ready())
+            resident = std::unique_lock<std::mutex>(resident_busy[S->device], std::try_to_lock);
+        if (resident.owns_lock()) {
+            // every tile resident: whole iterations in one launch.  The host looks at the stop flag as
+            // often as the caller asks, otherwise every kResidentIterations (a launch costs less than
+            // one of them, and each ends on state buffer 0)
+            int every = rp->check_every > 0 ? rp->check_every : kResidentIterations;
+            every += every & 1;
+            E3D_CUDA(cudaEventRecord(S->ev0, S->stream));
+            for (int left = max_iter; left > 0;) {
+                const int n = std::min(every, left);
+                S->launch_resident(n);
+                launches++;
+                left -= n;
+                E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, S->stream));
+                E3D_CUDA(cudaStreamSynchronize(S->stream));
+                if (S->ctl_host->done || S->ctl_host->fault) break;
+                if (left == 0) throw Error(E3D_ERR_TIMEOUT, "run did not reach its stop condition");
+            }
+        } else if (rp->profile_stages != 1) {
             int every = rp->check_every > 0 ? rp->check_every : 32;
             every += every & 1;  // whole graphs start and end on buffer 0
             const bool timed = rp->profile_stages == 2;

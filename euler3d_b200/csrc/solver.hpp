@@ -9,7 +9,9 @@
 
 #include "common.hpp"
 #include "euler3d_b200.h"
+#include "reduce.cuh"
 #include "stage.cuh"
+#include "stage_resident.cuh"
 
 namespace e3d {
 
@@ -27,9 +29,13 @@ void launch_colour_fast(const StageArgs &a, const ColourFace *faces, int n, doub
 void launch_colour_finish_fast(const StageArgs &a, const double2 *rc, cudaStream_t s);
 struct Solver;
 void build_colours(Solver *S);
+int resident_max_blocks_exact(int shape, size_t smem);
+int resident_max_blocks_fast(int shape, size_t smem);
+int resident_max_blocks_f32(int shape, size_t smem);
+void launch_resident_exact(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
+void launch_resident_fast(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
+void launch_resident_f32(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
 
-constexpr int kReduceThreads = 256;
-constexpr int kCoeffThreads = 512;
 void launch_update_exact(const StageArgs &a, cudaStream_t s);
 void launch_fast_reciprocals(const double *x, int64_t n, double *out, cudaStream_t s);
 void launch_update_fast(const StageArgs &a, cudaStream_t s);
@@ -42,36 +48,6 @@ void launch_batch_f32(const BatchStage &bs, int grid, size_t smem_bytes, cudaStr
 void launch_batch_ws_exact(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
 void launch_batch_ws_fast(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
 void launch_batch_ws_f32(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
-
-struct CoeffArgs {
-    int n_wall;
-    const int *__restrict__ cell;       // device cell of each wall face, reference wall order
-    const double *__restrict__ svec;    // 3 per wall face: full face normal
-    const double *__restrict__ center;  // 3 per wall face: face centre
-    const double2 *__restrict__ q;
-    const double *__restrict__ w0;      // FP32_FLUX mode: pressure from the double conservative state
-    int w0_stride;
-    double gamma;
-    double p_inf, cp_factor, cref, sref, ref[3];
-    int axis[3], sign[3];
-    Control *ctl;
-    int run_mode;                       // 1: sampled inside e3d_solver_run, apply the stop test
-    int sequential;                     // 1: sum in the reference's wall order (FP64_EXACT)
-    double *__restrict__ out;           // 6 doubles (force, moment) when not in run mode
-    double *__restrict__ cp_out;        // [n_wall] Cp of every wall face (AeroCoefficients::_cp), or null
-    double *__restrict__ samples;       // run mode: 7 doubles (iteration, force, moment) per sample, or null
-};
-
-// Arguments of the RMS / stop-test kernel of one solver.
-struct FinalizeArgs {
-    const double *partials;  // per-tile (per-block) sums of R_rho^2
-    int n_part;
-    double n_domain;         // interior cells
-    double *hist;            // RMS history
-    Control *ctl;
-    const double *rsq;       // FP64_EXACT: R_rho^2 per cell in reference order, summed sequentially
-    int n_cells;
-};
 
 // Residual smoothing (EulerSolver::smoothResiduals, src/solver/EulerSolver.cpp:483-518): one Jacobi
 // pass over every cell.
@@ -91,7 +67,7 @@ struct SmoothArgs {
 // Kernels of solver.cu, launched through these.
 void launch_finalize(const FinalizeArgs &f, cudaStream_t s);
 void launch_coeff(const CoeffArgs &c, cudaStream_t s);
-void launch_finalize_batch(const FinalizeArgs *f, const int *n_members, int grid, cudaStream_t s);
+void launch_finalize_batch(const FinalizeArgs *f, const int *n_members, int grid, bool exact, cudaStream_t s);
 void launch_coeff_batch(const CoeffArgs *c, const int *n_members, int parity, int grid, cudaStream_t s);
 void launch_control_gather(Control *const *ctl, const int *n_members, Control *out, int grid, cudaStream_t s);
 void launch_smooth(const SmoothArgs &a, cudaStream_t s);
@@ -199,6 +175,8 @@ struct Solver {
         tile_rec32_off.release();
         tile_contrib.release();
         release_colours();
+        resident_flags.release();
+        resident_words.release();
         cf.release();
         fgeo.release();
         cgeo.release();
@@ -245,6 +223,7 @@ struct Solver {
                (int64_t)(w0.n + ecell.n + minit.n + ghost.n + partials.n + staging.n + wall_svec.n + wall_center.n +
                          hist.n + scratch.n + den.n + rbuf.n + smooth_flags.n + samples.n + wall_cp.n + rsq.n) * 8 +
                (int64_t)(nb_ptr.n + nb.n) * 4 + (int64_t)colour_faces.n * 48 + (int64_t)colour_r.n * 16 +
+               (int64_t)resident_flags.n * 4 + (int64_t)resident_words.n * 16 +
                (int64_t)sizeof(Control);
     }
 
@@ -300,7 +279,80 @@ struct Solver {
         return a;
     }
 
+    // Resident kernel (stage_resident.cuh): its block shape, -1 when the tiles do not all fit on the
+    // GPU at once; the words its tiles exchange (allocated by the first resident run) and their tag.
+    int resident_shape = -1;
+    int max_far = 0;               // farfield and unclassified faces of a tile, at most
+    size_t resident_smem = 0;
+    DevBuf<unsigned> resident_flags;
+    DevBuf<uint4> resident_words;
+    unsigned resident_tag = 1;
+
+    // The largest block size at which every tile and the control block are resident together.
+    void plan_resident() {
+        if (!tiles_ok || smoothing) return;
+        const int prec = f32 ? PREC_F32 : prm.precision == E3D_PREC_FP64 ? PREC_FAST : PREC_EXACT;
+        size_t smem = resident_smem_bytes(prec, smem_cells, smem_faces, max_contrib, max_far, n_tiles);
+        // exact mode with a block per SM: room for R_rho^2 of every cell in the control block
+        const size_t with_rsq = std::max(smem, kControlHead + 8 * (size_t)N);
+        if (prec == PREC_EXACT && n_tiles < n_sm && with_rsq <= 226 * 1024) smem = with_rsq;
+        if (smem > 226 * 1024) return;
+        for (int shape = 0; shape < kResidentShapeCount; shape++) {
+            const int per_sm = prec == PREC_F32    ? resident_max_blocks_f32(shape, smem)
+                               : prec == PREC_FAST ? resident_max_blocks_fast(shape, smem)
+                                                   : resident_max_blocks_exact(shape, smem);
+            if ((int64_t)per_sm * n_sm < n_tiles + 1) continue;
+            resident_shape = shape;
+            resident_smem = smem;
+            return;
+        }
+    }
+
+    // A run with the resident kernel is possible and its buffers are there.
+    bool resident_ready() {
+        if (resident_shape < 0) return false;
+        if (resident_words.p) return true;
+        const size_t per_cell = f32 ? ResidentLayout<PREC_F32>::kWords : ResidentLayout<PREC_FAST>::kWords;
+        try {
+            if (!resident_flags.p) resident_flags.alloc((size_t)(n_tiles + kControlWords) * kFlagStride);
+            resident_words.alloc(2 * per_cell * (size_t)n_tiles * kTileCells + n_tiles);
+        } catch (const Error &) {  // no memory for it: the stage kernels need none
+            resident_words.p = nullptr;
+            resident_words.n = 0;
+            resident_shape = -1;
+            return false;
+        }
+        E3D_CUDA(cudaMemsetAsync(resident_words.p, 0, resident_words.n * sizeof(uint4), stream));
+        return true;
+    }
+
+    // `iters` iterations from state buffer 0 with the resident kernel.
+    void launch_resident(int iters) {
+        E3D_CUDA(cudaMemsetAsync(resident_flags.p, 0, resident_flags.n * sizeof(unsigned), stream));
+        const StageArgs a = stage_args(0, 0.0, 0, 0);
+        ResidentArgs r{};
+        r.flags = resident_flags.p;
+        r.partials = resident_words.p;
+        r.words = resident_words.p + n_tiles;
+        r.tag = resident_tag;
+        resident_tag += (unsigned)(iters * n_stages()) + 2;
+        for (int b = 0; b < 2; b++) {
+            r.q[b] = q[b].p;
+            r.q32[b] = q32[b].p;
+            r.coeff[b] = coeff_args(b, 1, nullptr);
+        }
+        r.iterations = iters;
+        r.stages = n_stages();
+        r.max_far = max_far;
+        r.stage_rsq = resident_smem >= kControlHead + 8 * (size_t)N;
+        r.fin = finalize_args(partials.p, hist.p);
+        if (f32) launch_resident_f32(a, r, resident_shape, resident_smem, stream);
+        else if (prm.precision == E3D_PREC_FP64) launch_resident_fast(a, r, resident_shape, resident_smem, stream);
+        else launch_resident_exact(a, r, resident_shape, resident_smem, stream);
+    }
+
     int variant = 0;                // stage-kernel variant picked by autotune()
+    bool variant_forced = false;    // by e3d_run_params.stage_kernel: later runs keep it
     float variant_ms[kStageVariants] = {};
 
     // Variants compiled for this precision and possible on this mesh.  FP32_FLUX mode has face-tile

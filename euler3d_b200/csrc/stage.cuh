@@ -122,6 +122,24 @@ struct StageArgs {
                                      // stage (the residual phase of a split last stage)
 };
 
+// What changes from stage to stage of a run, beside the state that is read: a stage kernel reads it from
+// its arguments where it is used, the resident kernel (stage_resident.cuh) has it in its own loop.
+struct ArgStep {
+    const StageArgs &a;
+    __device__ __forceinline__ double alpha() const { return a.alpha; }
+    __device__ __forceinline__ bool first_stage() const { return a.first_stage; }
+    __device__ __forceinline__ bool last_stage() const { return a.last_stage; }
+    // wall / symmetry ghost records are written
+    __device__ __forceinline__ bool ghost_store() const { return a.last_stage || a.residual_only || a.ghost_out; }
+    // the loaded interior Mach still holds
+    __device__ __forceinline__ bool minit_valid() const { return a.ctl->minit_valid; }
+    // record of the ghost cell behind boundary face j of the tile
+    __device__ __forceinline__ double *ghost(int, int slot, int) const { return a.ghost + 8 * (size_t)slot; }
+    __device__ __forceinline__ bool stores_state() const { return true; }
+    __device__ __forceinline__ double2 *qout() const { return a.qout; }
+    __device__ __forceinline__ float4 *q32out() const { return a.q32out; }
+};
+
 // One face of a tile: code = l | r << 10 | tag << 20 (local cell indices; r unused for boundary
 // faces), ghost slot for boundary faces, unit normal and area.
 struct FaceRec {
@@ -407,20 +425,32 @@ __device__ __forceinline__ void ghost_store(double *gp, double rho, double u, do
     g2[3] = make_double2(H, M);
 }
 
-// Tail shared by subsonic farfield, wall and symmetry ghosts (src/solver/PhysicalBC.cpp:62-66).
-__device__ __forceinline__ void ghost_finish(double *gp, double g, double rho, double u, double v, double w,
-                                             double p, double c, Prim &out) {
-    double q2 = u * u + v * v + w * w;
-    double M = sqrt(q2) / c;
-    double E = p / ((g - 1) * rho) + (q2 / 2.0);
-    double H = E + (p / rho);
-    ghost_store(gp, rho, u, v, w, p, E, H, M);
-    out = Prim{rho, u, v, w, p, H};
-}
-
 // Arithmetic of a stage kernel: the reference's own operations, restructured double precision, or
 // single-precision fluxes.
 enum : int { PREC_EXACT = 0, PREC_FAST = 1, PREC_F32 = 2 };
+
+// Tail shared by subsonic farfield, wall and symmetry ghosts (src/solver/PhysicalBC.cpp:62-66); c is the
+// interior cell's sound speed in exact mode and its reciprocal otherwise (two fast reciprocals and a
+// root instead of three divisions and a root).
+template <int PREC>
+__device__ __forceinline__ void ghost_finish(double *gp, double g, double rho, double u, double v, double w,
+                                             double p, double c, Prim &out) {
+    double M, E, H;
+    if (PREC == PREC_EXACT) {
+        double q2 = u * u + v * v + w * w;
+        M = sqrt(q2) / c;
+        E = p / ((g - 1) * rho) + (q2 / 2.0);
+        H = E + (p / rho);
+    } else {
+        const double q2 = fma(u, u, fma(v, v, w * w));
+        const double e = p * rcp_nr((g - 1.0) * rho);  // internal energy; p / rho = (gamma - 1) e
+        M = q2 == 0.0 ? 0.0 : q2 * rsqrt_nr(q2) * c;
+        E = fma(0.5, q2, e);
+        H = fma(g - 1.0, e, E);
+    }
+    ghost_store(gp, rho, u, v, w, p, E, H, M);
+    out = Prim{rho, u, v, w, p, H};
+}
 
 // BC::Wall / BC::Symmetry (src/solver/PhysicalBC.cpp:124-231): mirrored velocity.  The kernels
 // never read a wall or symmetry ghost back (it is rebuilt from its interior cell at every stage), so
@@ -436,8 +466,8 @@ __device__ __forceinline__ void ghost_mirror(double *gp, double g, const Prim &d
     double v = d.v - 2 * V * ny;
     double w = d.w - 2 * V * nz;
     if (store) {
-        double c = sqrt(g * (d.p / d.rho));
-        ghost_finish(gp, g, d.rho, u, v, w, d.p, c, out);
+        const double c = PREC == PREC_EXACT ? sqrt(g * (d.p / d.rho)) : d.rho * rsqrt_nr(g * d.p * d.rho);
+        ghost_finish<PREC>(gp, g, d.rho, u, v, w, d.p, c, out);
     } else {
         double H = 0.0;
         if (need_h) {  // ghost_finish's E and H, in its operation order
@@ -454,39 +484,63 @@ __device__ __forceinline__ void ghost_mirror(double *gp, double g, const Prim &d
 }
 
 // Farfield ghost (EulerSolver::updateBC, src/solver/EulerSolver.cpp:205-227): the branch comes
-// from the ghost's previous Mach and normal velocity; d_M / d_E are the interior Mach and energy.
+// from the ghost's previous Mach and normal velocity; mach() and energy() give the interior cell's Mach
+// and energy where the branch needs them.  Outside the exact mode 1/rho and 1/c are formed once.
+template <int PREC, typename MACH, typename ENERGY>
 __device__ __forceinline__ void ghost_farfield(double *gp, double g, const Freestream &fs, const Prim &d,
-                                               double d_M, double d_E, double nx, double ny, double nz,
+                                               MACH &&mach, ENERGY &&energy, double nx, double ny, double nz,
                                                Prim &out) {
     double2 gu = reinterpret_cast<const double2 *>(gp)[0];
     double2 gv = reinterpret_cast<const double2 *>(gp)[1];
     double gM = gp[7];
     double V = gu.y * nx + gv.x * ny + gv.y * nz;
     if (gM >= 1.0 && V > 0.0) {  // BC::FarfieldSupersonicOutflow, PhysicalBC.cpp:26-40
-        ghost_store(gp, d.rho, d.u, d.v, d.w, d.p, d_E, d.H, d_M);
+        ghost_store(gp, d.rho, d.u, d.v, d.w, d.p, energy(), d.H, mach());
         out = d;
-    } else if (gM < 1.0 && V > 0.0) {  // BC::FarfieldSubsonicOutflow, PhysicalBC.cpp:82-121
-        double c = sqrt(g * (d.p / d.rho));
-        double p = fs.p;
-        double rho = d.rho + (p - d.p) / (c * c);
-        double u = d.u + nx * (d.p - p) / (d.rho * c);
-        double v = d.v + ny * (d.p - p) / (d.rho * c);
-        double w = d.w + nz * (d.p - p) / (d.rho * c);
-        ghost_finish(gp, g, rho, u, v, w, p, c, out);
     } else if (gM >= 1.0 && V <= 0.0) {  // BC::FarfieldSupersonicInflow, PhysicalBC.cpp:11-23
         ghost_store(gp, fs.rho, fs.u, fs.v, fs.w, fs.p, fs.E, fs.H, fs.M);
         out = Prim{fs.rho, fs.u, fs.v, fs.w, fs.p, fs.H};
-    } else if (gM < 1.0 && V <= 0.0) {  // BC::FarfieldSubsonicInflow, PhysicalBC.cpp:43-79
-        double c = sqrt(g * (d.p / d.rho));
-        double p = 0.5 * (fs.p + d.p - d.rho * c * ((nx * (fs.u - d.u)) + (ny * (fs.v - d.v)) + (nz * (fs.w - d.w))));
-        double rho = fs.rho + (p - fs.p) / (c * c);
-        double u = fs.u - nx * (fs.p - p) / (d.rho * c);
-        double v = fs.v - ny * (fs.p - p) / (d.rho * c);
-        double w = fs.w - nz * (fs.p - p) / (d.rho * c);
-        ghost_finish(gp, g, rho, u, v, w, p, c, out);
-    } else {  // NaN Mach or velocity: the reference leaves the ghost as it is
+    } else if (!(gM < 1.0 && (V > 0.0 || V <= 0.0))) {  // NaN Mach or velocity: the reference leaves the ghost as it is
         double2 gph = reinterpret_cast<const double2 *>(gp)[2];
         out = Prim{gu.x, gu.y, gv.x, gv.y, gph.x, gp[6]};
+    } else if (PREC == PREC_EXACT) {
+        const double c = sqrt(g * (d.p / d.rho));
+        double p, rho, u, v, w;
+        if (V > 0.0) {  // BC::FarfieldSubsonicOutflow, PhysicalBC.cpp:82-121
+            p = fs.p;
+            rho = d.rho + (p - d.p) / (c * c);
+            u = d.u + nx * (d.p - p) / (d.rho * c);
+            v = d.v + ny * (d.p - p) / (d.rho * c);
+            w = d.w + nz * (d.p - p) / (d.rho * c);
+        } else {  // BC::FarfieldSubsonicInflow, PhysicalBC.cpp:43-79
+            p = 0.5 * (fs.p + d.p - d.rho * c * ((nx * (fs.u - d.u)) + (ny * (fs.v - d.v)) + (nz * (fs.w - d.w))));
+            rho = fs.rho + (p - fs.p) / (c * c);
+            u = fs.u - nx * (fs.p - p) / (d.rho * c);
+            v = fs.v - ny * (fs.p - p) / (d.rho * c);
+            w = fs.w - nz * (fs.p - p) / (d.rho * c);
+        }
+        ghost_finish<PREC>(gp, g, rho, u, v, w, p, c, out);
+    } else {
+        // with r = 1 / sqrt(gamma p rho): 1/c = rho r, 1/(rho c) = r, rho c = gamma p rho r
+        const double gpr = g * d.p * d.rho, r = rsqrt_nr(gpr), ic = d.rho * r;
+        double p, rho, u, v, w;
+        if (V > 0.0) {
+            const double dpr = (d.p - fs.p) * r;
+            p = fs.p;
+            rho = fma(p - d.p, ic * ic, d.rho);
+            u = fma(nx, dpr, d.u);
+            v = fma(ny, dpr, d.v);
+            w = fma(nz, dpr, d.w);
+        } else {
+            const double dV = fma(nx, fs.u - d.u, fma(ny, fs.v - d.v, nz * (fs.w - d.w)));
+            p = 0.5 * (fs.p + d.p - gpr * r * dV);
+            const double dpr = (p - fs.p) * r;
+            rho = fma(p - fs.p, ic * ic, fs.rho);
+            u = fma(nx, dpr, fs.u);
+            v = fma(ny, dpr, fs.v);
+            w = fma(nz, dpr, fs.w);
+        }
+        ghost_finish<PREC>(gp, g, rho, u, v, w, p, ic, out);
     }
 }
 
@@ -501,8 +555,10 @@ __device__ __forceinline__ void ghost_flux(const Prim &s, double nx, double ny, 
 }
 
 // ------------------------------------------------------------------------------ shared pieces
+// Sum of v over the block (a shuffle tree per warp, then one over the warps), to thread 0; includes a
+// barrier.  Threads beyond kStageThreads pass 0, so the sum has the same bits for every block size.
 template <int NT = kStageThreads>
-__device__ __forceinline__ void block_sum_store(double v, double *dst) {
+__device__ __forceinline__ double block_sum(double v) {
     __shared__ double warp_sums[NT / 32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -513,8 +569,14 @@ __device__ __forceinline__ void block_sum_store(double v, double *dst) {
         v = lane < NT / 32 ? warp_sums[lane] : 0.0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) *dst = v;
     }
+    return v;
+}
+
+template <int NT = kStageThreads>
+__device__ __forceinline__ void block_sum_store(double v, double *dst) {
+    v = block_sum<NT>(v);
+    if (threadIdx.x == 0) *dst = v;
 }
 
 // Boundary face of interior cell c (state me): updates its ghost cell (EulerSolver::updateBC,
@@ -522,11 +584,11 @@ __device__ __forceinline__ void block_sum_store(double v, double *dst) {
 // :331-339; farfield / unclassified: physical flux of the ghost, :349-357) and returns false, or
 // leaves the mirrored ghost in gs and returns true (symmetry: Roe against the ghost, :343-346).  The
 // FP64 mode forms the symmetry flux here too and always returns false.
-template <int PREC>
-__device__ __forceinline__ bool boundary_face(const StageArgs &a, int tag, double *gp, int c, const Prim &me,
-                                              const double4 &fg, double F[5], Prim &gs) {
+template <int PREC, typename STEP>
+__device__ __forceinline__ bool boundary_face(const StageArgs &a, const STEP &sp, int tag, double *gp, int c,
+                                              const Prim &me, const double4 &fg, double F[5], Prim &gs) {
     const double g = a.gamma;
-    const bool store = a.last_stage || a.residual_only || a.ghost_out;
+    const bool store = sp.ghost_store();
     if (tag == TAG_WALL) {
         ghost_mirror<PREC>(gp, g, me, fg.x, fg.y, fg.z, gs, store, false);
         F[0] = 0;
@@ -543,12 +605,14 @@ __device__ __forceinline__ bool boundary_face(const StageArgs &a, int tag, doubl
         return false;
     }
     if (tag == TAG_FAR) {
-        double q2 = me.u * me.u + me.v * me.v + me.w * me.w;
         // interior Mach as FlowField stores it (c/|u|, FlowField.cpp:157) unless the loaded state's
         // still holds; E is exact at stage 1 (ecell), recomputed from H at later stages
-        double dM = (a.first_stage && a.ctl->minit_valid) ? a.minit[c] : sqrt(g * (me.p / me.rho)) / sqrt(q2);
-        double dE = a.first_stage ? a.ecell[c] : me.H - me.p / me.rho;
-        ghost_farfield(gp, g, a.fs, me, dM, dE, fg.x, fg.y, fg.z, gs);
+        auto mach = [&] {
+            double q2 = me.u * me.u + me.v * me.v + me.w * me.w;
+            return sp.first_stage() && sp.minit_valid() ? a.minit[c] : sqrt(g * (me.p / me.rho)) / sqrt(q2);
+        };
+        auto energy = [&] { return sp.first_stage() ? a.ecell[c] : me.H - me.p / me.rho; };
+        ghost_farfield<PREC>(gp, g, a.fs, me, mach, energy, fg.x, fg.y, fg.z, gs);
     } else {  // unclassified boundary: the ghost keeps its (freestream) state
         double2 g0 = reinterpret_cast<const double2 *>(gp)[0];
         double2 g1 = reinterpret_cast<const double2 *>(gp)[1];
@@ -560,10 +624,12 @@ __device__ __forceinline__ bool boundary_face(const StageArgs &a, int tag, doubl
 }
 
 // Time step, Runge-Kutta update and primitive recovery of cell c from its residual R, the cell's
-// W0 and geometry; returns this cell's R_rho^2 on the last stage (for the RMS), else 0.
-template <bool EXACT>
-__device__ __forceinline__ double finish_cell(const StageArgs &a, int c, const Prim &me, double r_me,
-                                              const double R[5], const double W0[5], const double4 cg) {
+// W0 and geometry; returns this cell's R_rho^2 on the last stage (for the RMS), else 0.  The new state
+// is left in s and, on the last stage, the next step's W0 in W0.
+template <bool EXACT, typename STEP>
+__device__ __forceinline__ double finish_cell(const StageArgs &a, const STEP &sp, int c, const Prim &me,
+                                              double r_me, const double R[5], double W0[5], const double4 cg,
+                                              Prim &s) {
     const double g = a.gamma;
     // local time step, TimeStepMethod2 (src/solver/TimeIntegration.cpp:8-40)
     double lam, dt;
@@ -608,13 +674,12 @@ __device__ __forceinline__ double finish_cell(const StageArgs &a, int c, const P
     } else if (EXACT) {
         // W = W0 - alpha dt R / V and primitive recovery (EulerSolver.cpp:461-470, FlowField.cpp:140-171)
 #pragma unroll
-        for (int k = 0; k < 5; k++) W[k] = W0[k] - a.alpha * dt * R[k] / cg.w;
+        for (int k = 0; k < 5; k++) W[k] = W0[k] - sp.alpha() * dt * R[k] / cg.w;
     } else {
-        double coef = a.alpha * a.cfl * rcp_nr(lam);  // alpha dt / V
+        double coef = sp.alpha() * a.cfl * rcp_nr(lam);  // alpha dt / V
 #pragma unroll
         for (int k = 0; k < 5; k++) W[k] = fma(-coef, R[k], W0[k]);
     }
-    Prim s;
     double E;
     s.rho = W[0];
     if (EXACT) {
@@ -634,22 +699,21 @@ __device__ __forceinline__ double finish_cell(const StageArgs &a, int c, const P
         s.p = (g - 1.0) * fma(-0.5, fma(W[1], s.u, fma(W[2], s.v, W[3] * s.w)), W[4]);
         s.H = (W[4] + s.p) * ir;
     }
-    store_prim_cs(a.qout, c, s);
-    if (!a.last_stage) return 0.0;
+    if (sp.stores_state()) store_prim_cs(sp.qout(), c, s);
+    if (!sp.last_stage()) return 0.0;
     const size_t st = (size_t)a.w0_stride;
     if (a.integrator == E3D_INTEGRATOR_EULER) {  // the conservative state itself carries over
 #pragma unroll
-        for (int k = 0; k < 5; k++) __stcs(a.w0 + k * st + c, W[k]);
-        __stcs(a.ecell + c, E);
-        if (a.rsq) a.rsq[a.new2old[c]] = R[0] * R[0];
-        return R[0] * R[0];
+        for (int k = 0; k < 5; k++) W0[k] = W[k];
+    } else {  // the next step's W0 from the primitives (EulerSolver.cpp:431-438)
+        W0[0] = s.rho;
+        W0[1] = s.u * s.rho;
+        W0[2] = s.v * s.rho;
+        W0[3] = s.w * s.rho;
+        W0[4] = E * s.rho;
     }
-    // the next step's W0 from the primitives (EulerSolver.cpp:431-438)
-    __stcs(a.w0 + 0 * st + c, s.rho);
-    __stcs(a.w0 + 1 * st + c, s.u * s.rho);
-    __stcs(a.w0 + 2 * st + c, s.v * s.rho);
-    __stcs(a.w0 + 3 * st + c, s.w * s.rho);
-    __stcs(a.w0 + 4 * st + c, E * s.rho);
+#pragma unroll
+    for (int k = 0; k < 5; k++) __stcs(a.w0 + k * st + c, W0[k]);
     __stcs(a.ecell + c, E);
     if (a.rsq) a.rsq[a.new2old[c]] = R[0] * R[0];
     return R[0] * R[0];
@@ -664,6 +728,7 @@ __global__ void __launch_bounds__(kStageThreads, MINB) stage_kernel(StageArgs a)
     if (!a.residual_only && a.ctl->done) return;  // uniform across the grid
     const int c = blockIdx.x * kStageThreads + threadIdx.x;
     const double g = a.gamma;
+    const ArgStep sp{a};
     double r2 = 0.0;
     if (c < a.n_cells) {
         const Prim me = load_prim(a.qin, c);
@@ -697,7 +762,7 @@ __global__ void __launch_bounds__(kStageThreads, MINB) stage_kernel(StageArgs a)
                 }
             } else {
                 Prim gs;
-                roe = boundary_face<EXACT ? PREC_EXACT : PREC_FAST>(a, tag, a.ghost + 8 * (size_t)idx, c, me, fg, F, gs);
+                roe = boundary_face<EXACT ? PREC_EXACT : PREC_FAST>(a, sp, tag, a.ghost + 8 * (size_t)idx, c, me, fg, F, gs);
                 fl = me;
                 fr = gs;  // symmetry ghost
             }
@@ -716,7 +781,8 @@ __global__ void __launch_bounds__(kStageThreads, MINB) stage_kernel(StageArgs a)
         double W0[5];
 #pragma unroll
         for (int k = 0; k < 5; k++) W0[k] = a.w0[(size_t)k * a.w0_stride + c];
-        r2 = finish_cell<EXACT>(a, c, me, r_me, R, W0, a.cgeo[c]);
+        Prim out;
+        r2 = finish_cell<EXACT>(a, sp, c, me, r_me, R, W0, a.cgeo[c], out);
     }
     if (a.last_stage && !a.residual_only) block_sum_store(r2, a.partials + blockIdx.x);
 }
@@ -783,7 +849,7 @@ __global__ void __launch_bounds__(NT) colour_kernel(StageArgs a, const ColourFac
         return;
     }
     Prim gs;
-    boundary_face<PREC_FAST>(a, cf.tag, a.ghost + 8 * (size_t)cf.r, cf.l, L, fg, F, gs);
+    boundary_face<PREC_FAST>(a, ArgStep{a}, cf.tag, a.ghost + 8 * (size_t)cf.r, cf.l, L, fg, F, gs);
     colour_add(rc, cf.l, F, fg.w, true);
 }
 
@@ -803,7 +869,8 @@ __global__ void __launch_bounds__(kStageThreads) colour_finish_kernel(StageArgs 
         double W0[5];
 #pragma unroll
         for (int k = 0; k < 5; k++) W0[k] = a.w0[k * st + c];
-        r2 = finish_cell<false>(a, c, me, rsqrt_nr(a.gamma * me.p * me.rho), R, W0, a.cgeo[c]);
+        Prim out;
+        r2 = finish_cell<false>(a, ArgStep{a}, c, me, rsqrt_nr(a.gamma * me.p * me.rho), R, W0, a.cgeo[c], out);
     }
     if (a.last_stage && !a.residual_only) block_sum_store(r2, a.partials + blockIdx.x);
 }
@@ -943,14 +1010,15 @@ __device__ __forceinline__ Prim tile_prim(const double2 *st, int i) {
     return Prim{x.x, x.y, y.x, y.y, z.x, z.y};
 }
 
-// One flux per tile face; F*S of face j replaces record j (fs[5 j + k] aliases b.rec[j]).  Roots of
+// One flux per tile face j0, j0 + NT, ... below nf; F*S of face j goes to fs[5 j + k], which in the
+// one-block-per-tile kernels is record j itself.  Roots of
 // the face's states are taken per face: a per-cell pass over the tile before the fluxes would cost a
 // barrier phase and 16 bytes of shared memory per local cell, and measured slower on B200.
-template <bool EXACT, int NT>
-__device__ __forceinline__ void tile_fluxes(const StageArgs &a, const TileBuf &b, double *fs, int nf, int c0,
-                                            int tid) {
+template <bool EXACT, int NT, typename STEP>
+__device__ __forceinline__ void tile_fluxes(const StageArgs &a, const STEP &sp, const TileBuf &b, double *fs,
+                                            int j0, int nf, int c0) {
     const double g = a.gamma;
-    for (int j = tid; j < nf; j += NT) {
+    for (int j = j0; j < nf; j += NT) {
         const FaceRec fr = b.rec[j];
         const int l = fr.code & ((1 << kTileLocalBits) - 1);
         const int r = (fr.code >> kTileLocalBits) & ((1 << kTileLocalBits) - 1);
@@ -969,8 +1037,8 @@ __device__ __forceinline__ void tile_fluxes(const StageArgs &a, const TileBuf &b
             }
         } else {
             Prim gs;
-            double *gp = a.ghost + 8 * (size_t)fr.ghost;
-            if (boundary_face<EXACT ? PREC_EXACT : PREC_FAST>(a, tag, gp, c0 + l, L, fg, F, gs)) {
+            double *gp = sp.ghost(j, fr.ghost, tag);
+            if (boundary_face<EXACT ? PREC_EXACT : PREC_FAST>(a, sp, tag, gp, c0 + l, L, fg, F, gs)) {
                 // exact mode's symmetry face: the general flux against the mirrored ghost
                 if (a.scheme == 1) ausm_exact(L, gs, fg.x, fg.y, fg.z, g, F);
                 else roe_exact(L, gs, fg.x, fg.y, fg.z, g, F);
@@ -1000,9 +1068,10 @@ __device__ __forceinline__ void tile_load_cell(const StageArgs &a, int c0, int i
 // Cell i of the tile: sum of its contributions, then time step and update; returns R_rho^2 on
 // the last stage.  W0 and the geometry come from the caller, which loads them before the barrier
 // that ends the flux phase so that their latency overlaps the wait.
-template <bool EXACT>
-__device__ __forceinline__ double tile_update(const StageArgs &a, const TileBuf &b, const double *fs, int c0, int i,
-                                              const double W0[5], const double4 &cg) {
+template <bool EXACT, typename STEP>
+__device__ __forceinline__ double tile_update(const StageArgs &a, const STEP &sp, const TileBuf &b,
+                                              const double *fs, int c0, int i, double W0[5], const double4 &cg,
+                                              Prim &out) {
     const int T = kTileCells;
     double R[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     unsigned short e[6];
@@ -1019,7 +1088,7 @@ __device__ __forceinline__ double tile_update(const StageArgs &a, const TileBuf 
 #pragma unroll
         for (int q = 0; q < 5; q++) R[q] = fma(sg, fs[5 * j + q], R[q]);
     }
-    return finish_cell<EXACT>(a, c0 + i, me, EXACT ? 0.0 : rsqrt_nr(a.gamma * me.p * me.rho), R, W0, cg);
+    return finish_cell<EXACT>(a, sp, c0 + i, me, EXACT ? 0.0 : rsqrt_nr(a.gamma * me.p * me.rho), R, W0, cg, out);
 }
 
 // Bounded wait on an mbarrier phase by every thread (a.wait_polls polls); on timeout the fault word
@@ -1079,13 +1148,15 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, int tile, double *
         tile_drain(bar, 0);
         return;
     }
-    tile_fluxes<EXACT, kStageThreads>(a, b, fs, nf, c0, threadIdx.x);
+    const ArgStep sp{a};
+    tile_fluxes<EXACT, kStageThreads>(a, sp, b, fs, threadIdx.x, nf, c0);
     double W0[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     double4 cg = make_double4(0.0, 0.0, 0.0, 0.0);
     if ((int)threadIdx.x < nloc) tile_load_cell(a, c0, threadIdx.x, W0, cg);
     __syncthreads();
     double r2 = 0.0;
-    if ((int)threadIdx.x < nloc) r2 = tile_update<EXACT>(a, b, fs, c0, threadIdx.x, W0, cg);
+    Prim out;
+    if ((int)threadIdx.x < nloc) r2 = tile_update<EXACT>(a, sp, b, fs, c0, threadIdx.x, W0, cg, out);
     if (a.last_stage && !a.residual_only) block_sum_store(r2, partial);
 }
 
@@ -1163,7 +1234,8 @@ __global__ void __launch_bounds__(kStageThreads) update_kernel(StageArgs a) {
             W0[k] = a.w0[k * st + c];
         }
         const double r_me = EXACT ? 0.0 : rsqrt_nr(a.gamma * me.p * me.rho);
-        r2 = finish_cell<EXACT>(a, c, me, r_me, R, W0, a.cgeo[c]);
+        Prim out;
+        r2 = finish_cell<EXACT>(a, ArgStep{a}, c, me, r_me, R, W0, a.cgeo[c], out);
     }
     if (a.last_stage) block_sum_store(r2, a.partials + blockIdx.x);
 }

@@ -28,11 +28,19 @@ __device__ __forceinline__ float rsqrt_f(float x) {
 }
 
 // Cell record of a double-precision state (written by the update and by the state loader).
+__device__ __forceinline__ PrimF make_prim32(double rho, double u, double v, double w, double p, double H, double g) {
+    const float fr = (float)rho, fp = (float)p;
+    return PrimF{fr, (float)u, (float)v, (float)w, fp, (float)H, fr * rsqrt_f(fr), rsqrt_f((float)g * fp * fr)};
+}
+
+__device__ __forceinline__ void store_prim32(float4 *dst, const PrimF &s) {
+    __stcs(dst, make_float4(s.rho, s.u, s.v, s.w));  // streaming stores, as store_prim_cs
+    __stcs(dst + 1, make_float4(s.p, s.H, s.s, s.r));
+}
+
 __device__ __forceinline__ void make_rec32(float4 *dst, double rho, double u, double v, double w, double p, double H,
                                            double g) {
-    const float fr = (float)rho, fp = (float)p;
-    __stcs(dst, make_float4(fr, (float)u, (float)v, (float)w));  // streaming stores, as store_prim_cs
-    __stcs(dst + 1, make_float4(fp, (float)H, fr * rsqrt_f(fr), rsqrt_f((float)g * fp * fr)));
+    store_prim32(dst, make_prim32(rho, u, v, w, p, H, g));
 }
 
 // Roe flux with Harten's fix (Solver::Roe, src/solver/ConvectiveFluxesSchemes.cpp:10-165) in single
@@ -140,11 +148,13 @@ inline size_t tile32_smem_bytes(int smem_cells, int smem_faces, int max_contrib)
     return b + 16;
 }
 
-// One flux per tile face, threads tid, tid + nt, ...; F*S of face j replaces record j.
-__device__ __forceinline__ void tile_fluxes_f32(const StageArgs &a, const Tile32 &b, int nf, int c0, int tid, int nt) {
+// One flux per tile face j0, j0 + NT, ... below nf; F*S of face j goes to fs[6 j + k], which in the
+// one-block-per-tile kernels is record j itself.
+template <int NT, typename STEP>
+__device__ __forceinline__ void tile_fluxes_f32(const StageArgs &a, const STEP &sp, const Tile32 &b, float *fs,
+                                                int j0, int nf, int c0) {
     const float gf = (float)a.gamma;
-    float *fs = reinterpret_cast<float *>(b.rec);
-    for (int j = tid; j < nf; j += nt) {
+    for (int j = j0; j < nf; j += NT) {
         const FaceRec32 fr = b.rec[j];
         const int l = fr.code & ((1 << kTileLocalBits) - 1);
         const int r = (fr.code >> kTileLocalBits) & ((1 << kTileLocalBits) - 1);
@@ -159,7 +169,7 @@ __device__ __forceinline__ void tile_fluxes_f32(const StageArgs &a, const Tile32
             const double4 fg = make_double4(fr.nx, fr.ny, fr.nz, fr.S);
             double Fd[5];
             Prim gs;
-            if (boundary_face<PREC_F32>(a, tag, a.ghost + 8 * (size_t)fr.ghost, c0 + l, Ld, fg, Fd, gs)) {
+            if (boundary_face<PREC_F32>(a, sp, tag, sp.ghost(j, fr.ghost, tag), c0 + l, Ld, fg, Fd, gs)) {
                 const PrimF G{(float)gs.rho, (float)gs.u, (float)gs.v, (float)gs.w, (float)gs.p, (float)gs.H, L.s, L.r};
                 if (a.scheme == 1) ausm_f32(L, G, fr.nx, fr.ny, fr.nz, gf, F);
                 else roe_f32(L, G, fr.nx, fr.ny, fr.nz, gf, F);
@@ -183,11 +193,12 @@ __device__ __forceinline__ void tile_load_cell_f32(const StageArgs &a, int c, do
 }
 
 // Cell i of the tile: sum of its faces' F*S, time step and update; returns R_rho^2 on the last stage.
-__device__ __forceinline__ double tile_update_f32(const StageArgs &a, const Tile32 &b, int c0, int i, const double W0[5],
-                                                  const float4 &cg) {
+template <typename STEP>
+__device__ __forceinline__ double tile_update_f32(const StageArgs &a, const STEP &sp, const Tile32 &b,
+                                                  const float *fs, int c0, int i, double W0[5], const float4 &cg,
+                                                  PrimF &out) {
     const int T = kTileCells, MC = a.max_contrib;
     const float gf = (float)a.gamma;
-    const float *fs = reinterpret_cast<const float *>(b.rec);
     const PrimF me = prim32(b.st, i);
     double R[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     unsigned short e[6];
@@ -213,7 +224,7 @@ __device__ __forceinline__ double tile_update_f32(const StageArgs &a, const Tile
         return 0.0;
     }
     // W = W0 - alpha dt R / V in double (alpha dt / V = alpha cfl / lambda)
-    const double coef = a.alpha * a.cfl * rcp_nr((double)lam);
+    const double coef = sp.alpha() * a.cfl * rcp_nr((double)lam);
     double W[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) W[k] = fma(-coef, R[k], W0[k]);
@@ -221,12 +232,16 @@ __device__ __forceinline__ double tile_update_f32(const StageArgs &a, const Tile
     const double u = W[1] * ir, v = W[2] * ir, w = W[3] * ir;
     const double p = (a.gamma - 1.0) * fma(-0.5, fma(W[1], u, fma(W[2], v, W[3] * w)), W[4]);
     const double H = (W[4] + p) * ir;
-    make_rec32(a.q32out + 2 * (size_t)c, W[0], u, v, w, p, H, a.gamma);
-    if (!a.last_stage) return 0.0;
+    out = make_prim32(W[0], u, v, w, p, H, a.gamma);
+    if (sp.stores_state()) store_prim32(sp.q32out() + 2 * (size_t)c, out);
+    if (!sp.last_stage()) return 0.0;
     // the conservative state carries over exactly in double
     const size_t sd = (size_t)a.w0_stride;
 #pragma unroll
-    for (int k = 0; k < 5; k++) __stcs(a.w0 + k * sd + c, W[k]);
+    for (int k = 0; k < 5; k++) {
+        W0[k] = W[k];
+        __stcs(a.w0 + k * sd + c, W[k]);
+    }
     __stcs(a.ecell + c, W[4] * ir);
     return R[0] * R[0];
 }
@@ -282,14 +297,17 @@ __device__ __forceinline__ void tile_body_f32(const StageArgs &a, int tile, doub
         tile_drain(bar, 0);
         return;
     }
-    tile_fluxes_f32(a, b, nf, c0, threadIdx.x, kStageThreads);
+    const ArgStep sp{a};
+    float *fs = reinterpret_cast<float *>(b.rec);
+    tile_fluxes_f32<kStageThreads>(a, sp, b, fs, threadIdx.x, nf, c0);
     const int i = threadIdx.x;
     double W0[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     float4 cg = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < nloc) tile_load_cell_f32(a, c0 + i, W0, cg);  // latency overlaps the barrier's wait
     __syncthreads();
     double r2 = 0.0;
-    if (i < nloc) r2 = tile_update_f32(a, b, c0, i, W0, cg);
+    PrimF out;
+    if (i < nloc) r2 = tile_update_f32(a, sp, b, fs, c0, i, W0, cg, out);
     if (a.last_stage && !a.residual_only) block_sum_store(r2, partial);
 }
 

@@ -310,25 +310,29 @@ __device__ __forceinline__ void ws_body(const StageArgs &solo, const BatchStage 
         const bool run = !BATCH || !a.ctl->done;  // the member of a batch item may have stopped
         double r2 = 0.0;
         if (run) {
+            const ArgStep sp{a};
             const int c0 = tile * T, nloc = min(T, a.n_cells - c0);
             const int nf = meta[bi];  // the producer's, instead of a global-memory round trip
             if (F32) {
                 const Tile32 b = tile32_at(base + slot, a.smem_cells, a.smem_faces);
-                tile_fluxes_f32(a, b, nf, c0, tid, T);
+                float *fs = reinterpret_cast<float *>(b.rec);
+                tile_fluxes_f32<kTileCells>(a, sp, b, fs, tid, nf, c0);
                 double W0[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
                 float4 cg = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (tid < nloc) tile_load_cell_f32(a, c0 + tid, W0, cg);
                 named_sync(bar_id, T);
-                if (tid < nloc) r2 = tile_update_f32(a, b, c0, tid, W0, cg);
+                PrimF out;
+                if (tid < nloc) r2 = tile_update_f32(a, sp, b, fs, c0, tid, W0, cg, out);
             } else {
                 const TileBuf b = tile_buf_at(base + slot, a.smem_cells, a.smem_faces, a.max_contrib);
                 double *fs = reinterpret_cast<double *>(b.rec);
-                tile_fluxes<EXACT, kTileCells>(a, b, fs, nf, c0, tid);
+                tile_fluxes<EXACT, kTileCells>(a, sp, b, fs, tid, nf, c0);
                 double W0[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
                 double4 cg = make_double4(0.0, 0.0, 0.0, 0.0);
                 if (tid < nloc) tile_load_cell(a, c0, tid, W0, cg);
                 named_sync(bar_id, T);
-                if (tid < nloc) r2 = tile_update<EXACT>(a, b, fs, c0, tid, W0, cg);
+                Prim out;
+                if (tid < nloc) r2 = tile_update<EXACT>(a, sp, b, fs, c0, tid, W0, cg, out);
             }
         }
         const bool sum = run && a.last_stage && !a.residual_only;  // uniform across the group
