@@ -45,6 +45,23 @@ inline void raise_smem_limit(const void *func, size_t bytes) {
     cur = bytes;
 }
 
+// Launches a kernel as a programmatic dependent of the kernel before it on the stream: it may start
+// while that one runs and waits for it where it says pdl_wait (stage.cuh).
+template <typename... Params, typename... Args>
+void launch_dependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t s, Args &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    E3D_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+}
+
 // Runs fn and converts exceptions into an e3d_status plus the thread's last-error message.
 template <typename F>
 e3d_status guarded(F &&fn) {

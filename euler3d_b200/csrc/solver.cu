@@ -26,6 +26,8 @@ namespace e3d {
 template <int NT>
 __global__ void __launch_bounds__(NT) finalize_kernel(FinalizeArgs f) {
     __shared__ ControlScratch sh;
+    pdl_release();
+    pdl_wait();
     finalize_body<NT>(f, f.ctl, f.partials, sh);
 }
 
@@ -33,7 +35,10 @@ __global__ void __launch_bounds__(NT) finalize_kernel(FinalizeArgs f) {
 template <int NT>
 __global__ void __launch_bounds__(NT) finalize_batch_kernel(const FinalizeArgs *__restrict__ f,
                                                             const int *__restrict__ n_members) {
-    if ((int)blockIdx.x >= *n_members) return;
+    pdl_release();
+    const bool mine = (int)blockIdx.x < *n_members;
+    pdl_wait();
+    if (!mine) return;
     __shared__ ControlScratch sh;
     const FinalizeArgs a = f[blockIdx.x];
     finalize_body<NT>(a, a.ctl, a.partials, sh);
@@ -41,13 +46,18 @@ __global__ void __launch_bounds__(NT) finalize_batch_kernel(const FinalizeArgs *
 
 __global__ void __launch_bounds__(kCoeffThreads) coeff_kernel(CoeffArgs a) {
     __shared__ ControlScratch sh;
+    pdl_release();
+    pdl_wait();
     coeff_body<kCoeffThreads>(a, a.ctl, sh);
 }
 
 // Block m: member m of a batch, its arguments for the state buffer `parity`.
 __global__ void __launch_bounds__(kCoeffThreads) coeff_batch_kernel(const CoeffArgs *__restrict__ c,
                                                                     const int *__restrict__ n_members, int parity) {
-    if ((int)blockIdx.x >= *n_members) return;
+    pdl_release();
+    const bool mine = (int)blockIdx.x < *n_members;
+    pdl_wait();
+    if (!mine) return;
     __shared__ ControlScratch sh;
     const CoeffArgs a = c[2 * blockIdx.x + parity];
     coeff_body<kCoeffThreads>(a, a.ctl, sh);
@@ -130,16 +140,16 @@ void launch_smooth(const SmoothArgs &a, cudaStream_t s) {
 
 // FP64_EXACT's sum over every cell takes a larger block than the sum of the block partials.
 void launch_finalize(const FinalizeArgs &f, cudaStream_t s) {
-    if (f.rsq) finalize_kernel<kOrderedThreads><<<1, kOrderedThreads, 0, s>>>(f);
-    else finalize_kernel<kReduceThreads><<<1, kReduceThreads, 0, s>>>(f);
+    if (f.rsq) launch_dependent(finalize_kernel<kOrderedThreads>, 1, kOrderedThreads, 0, s, f);
+    else launch_dependent(finalize_kernel<kReduceThreads>, 1, kReduceThreads, 0, s, f);
 }
-void launch_coeff(const CoeffArgs &c, cudaStream_t s) { coeff_kernel<<<1, kCoeffThreads, 0, s>>>(c); }
+void launch_coeff(const CoeffArgs &c, cudaStream_t s) { launch_dependent(coeff_kernel, 1, kCoeffThreads, 0, s, c); }
 void launch_finalize_batch(const FinalizeArgs *f, const int *n_members, int grid, bool exact, cudaStream_t s) {
-    if (exact) finalize_batch_kernel<kOrderedThreads><<<grid, kOrderedThreads, 0, s>>>(f, n_members);
-    else finalize_batch_kernel<kReduceThreads><<<grid, kReduceThreads, 0, s>>>(f, n_members);
+    if (exact) launch_dependent(finalize_batch_kernel<kOrderedThreads>, grid, kOrderedThreads, 0, s, f, n_members);
+    else launch_dependent(finalize_batch_kernel<kReduceThreads>, grid, kReduceThreads, 0, s, f, n_members);
 }
 void launch_coeff_batch(const CoeffArgs *c, const int *n_members, int parity, int grid, cudaStream_t s) {
-    coeff_batch_kernel<<<grid, kCoeffThreads, 0, s>>>(c, n_members, parity);
+    launch_dependent(coeff_batch_kernel, grid, kCoeffThreads, 0, s, c, n_members, parity);
 }
 void launch_control_gather(Control *const *ctl, const int *n_members, Control *out, int grid, cudaStream_t s) {
     control_gather_kernel<<<grid, 64, 0, s>>>(ctl, n_members, out);
@@ -852,7 +862,6 @@ static void create_solver(const e3d_mesh_desc *d, const e3d_flow_params *p, Solv
     E3D_CUDA(cudaMemsetAsync(S->ctl, 0, sizeof(Control), s));
     E3D_CUDA(cudaEventCreate(&S->ev0));
     E3D_CUDA(cudaEventCreate(&S->ev1));
-    S->plan_resident();
     S->new2old = std::move(new2old);
     S->ghost_ref = std::move(ghost_ref);
     E3D_CUDA(cudaStreamSynchronize(s));

@@ -280,7 +280,9 @@ struct Solver {
     }
 
     // Resident kernel (stage_resident.cuh): its block shape, -1 when the tiles do not all fit on the
-    // GPU at once; the words its tiles exchange (allocated by the first resident run) and their tag.
+    // GPU at once, and the words its tiles exchange with their tag: planned and allocated by the first
+    // run that could use it (batch members never do).
+    bool resident_planned = false;
     int resident_shape = -1;
     int max_far = 0;               // farfield and unclassified faces of a tile, at most
     size_t resident_smem = 0;
@@ -290,6 +292,7 @@ struct Solver {
 
     // The largest block size at which every tile and the control block are resident together.
     void plan_resident() {
+        resident_planned = true;
         if (!tiles_ok || smoothing) return;
         const int prec = f32 ? PREC_F32 : prm.precision == E3D_PREC_FP64 ? PREC_FAST : PREC_EXACT;
         size_t smem = resident_smem_bytes(prec, smem_cells, smem_faces, max_contrib, max_far, n_tiles);
@@ -310,6 +313,7 @@ struct Solver {
 
     // A run with the resident kernel is possible and its buffers are there.
     bool resident_ready() {
+        if (!resident_planned) plan_resident();
         if (resident_shape < 0) return false;
         if (resident_words.p) return true;
         const size_t per_cell = f32 ? ResidentLayout<PREC_F32>::kWords : ResidentLayout<PREC_FAST>::kWords;

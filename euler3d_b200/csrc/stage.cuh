@@ -554,6 +554,17 @@ __device__ __forceinline__ void ghost_flux(const Prim &s, double nx, double ny, 
     F[4] = s.rho * s.H * V;
 }
 
+// ------------------------------------------------------------------------------ dependent launches
+// The kernels of an iteration follow one another as programmatic dependent launches: a block lets the
+// next kernel start as soon as it runs itself (pdl_release), so that kernel's first blocks take the SMs
+// that the last wave leaves free and do what needs no earlier result -- tile sizes, halo lists, member
+// arguments, the copies of face records and contribution lists -- before they wait for this kernel to
+// end (pdl_wait).  Every block waits before it reads or writes anything another kernel writes, and
+// before it returns, so a kernel that has ended means all earlier ones have.  Both are no-ops in a
+// kernel launched without the attribute.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------------------ shared pieces
 // Sum of v over the block (a shuffle tree per warp, then one over the warps), to thread 0; includes a
 // barrier.  Threads beyond kStageThreads pass 0, so the sum has the same bits for every block size.
@@ -880,7 +891,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)_
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;\n fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
@@ -976,24 +991,30 @@ __device__ __forceinline__ TileBuf tile_buf_at(unsigned char *base, int LC, int 
     return b;
 }
 
-// One thread issues the tile's bulk copies onto bar (expecting their byte count); nf and rec_off are
-// the tile's face count and record offset.
-__device__ __forceinline__ void tile_issue_bulk(const StageArgs &a, int tile, int nf, long long rec_off,
+// One thread issues the tile's bulk copies onto bar, which takes two arrivals (each expecting its own
+// copies' bytes): the mesh's own data first -- nf and rec_off are the tile's face count and record
+// offset -- and the states once the previous stage has written them.
+__device__ __forceinline__ void tile_issue_mesh(const StageArgs &a, int tile, int nf, long long rec_off,
                                                 const TileBuf &b, uint64_t *bar) {
     const int T = kTileCells, MC = a.max_contrib;
     const int c0 = tile * T, nloc = min(T, a.n_cells - c0);
-    const uint32_t b_state = (uint32_t)nloc * 48u;
     const uint32_t b_rec = round16(40u * (uint32_t)nf);
     const uint32_t b_w0 = round16((uint32_t)nloc * 8u);  // stays inside the padded rows
     const uint32_t b_cg = (uint32_t)nloc * 32u;
     const uint32_t b_ct = (uint32_t)MC * T * 2u;
-    mbar_expect_tx(bar, b_state + b_rec + b_ct);
+    mbar_expect_tx(bar, b_rec + b_ct);
     const uint64_t once = l2_evict_first();
-    bulk_g2s(b.st, a.qin + 3 * (size_t)c0, b_state, bar);
     bulk_g2s_hint(b.rec, a.tile_rec + rec_off, b_rec, bar, once);
     bulk_g2s_hint(b.ct, a.tile_contrib + (size_t)tile * MC * T, b_ct, bar, once);
     for (int k = 0; k < 5; k++) bulk_prefetch_l2(a.w0 + (size_t)k * a.w0_stride + c0, b_w0);
     bulk_prefetch_l2(a.cgeo + c0, b_cg);
+}
+
+__device__ __forceinline__ void tile_issue_state(const StageArgs &a, int tile, const TileBuf &b, uint64_t *bar) {
+    const int c0 = tile * kTileCells;
+    const uint32_t b_state = (uint32_t)min(kTileCells, a.n_cells - c0) * 48u;
+    mbar_expect_tx(bar, b_state);
+    bulk_g2s(b.st, a.qin + 3 * (size_t)c0, b_state, bar);
 }
 
 // Halo state i of the tile (global cell h) into st[nloc + i] with three 16-byte cp.async.
@@ -1107,6 +1128,12 @@ __device__ __forceinline__ void tile_drain(uint64_t *bar, uint32_t parity) {
     }
 }
 
+// Had the run stopped when the block started?  Before pdl_wait the kernel that stops a run may still be
+// running, so only "yes" is final (the flag is cleared by the host alone).
+__device__ __forceinline__ bool run_stopped(const StageArgs &a) {
+    return !a.residual_only && *(volatile const int *)&a.ctl->done;
+}
+
 // ---- one block per tile, all loads issued at the start (variant 2)
 // Shared memory: TileBuf (face fluxes over the records) | mbarrier
 // The body is shared by tile_kernel (one solver) and tile_batch_kernel (several solvers in one
@@ -1121,22 +1148,34 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, int tile, double *
 
     const int c0 = tile * T;
     const int nloc = min(T, a.n_cells - c0);
-    // Every load the copies depend on is issued before the first barrier, and none of them waits
-    // for another (the halo entries sit at a fixed stride per tile), so the copies start one
-    // memory latency after the block does.  The run's done flag is read alongside them.
+    // Every load the copies depend on is issued first, and none of them waits for another (the halo
+    // entries sit at a fixed stride per tile), so the copies start one memory latency after the block
+    // does.  All of it is the mesh's; the run's done flag and the states come after the wait for the
+    // previous kernel.
     const int *hrow = a.tile_halo + (size_t)tile * a.halo_stride;
     const int i0 = threadIdx.x, i1 = threadIdx.x + T;
     const int hx0 = i0 < a.halo_stride ? hrow[i0] : -1;
     const int hx1 = i1 < a.halo_stride ? hrow[i1] : -1;
     const int fp0 = a.tile_face_ptr[tile], fp1 = a.tile_face_ptr[tile + 1];
     const long long rec_off = a.tile_rec_off[tile];
-    const bool done = !a.residual_only && a.ctl->done;
     const int nf = fp1 - fp0;
 
-    if (threadIdx.x == 0) mbar_init(bar, 1);
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 2);
+        if (run_stopped(a)) mbar_arrive(bar);
+        else tile_issue_mesh(a, tile, nf, rec_off, b, bar);
+    }
+    pdl_wait();
+    const bool done = !a.residual_only && a.ctl->done;
+    if (threadIdx.x == 0) {
+        if (done) mbar_arrive(bar);
+        else tile_issue_state(a, tile, b, bar);
+    }
     __syncthreads();
-    if (done) return;  // uniform across the block (the run stopped: this stage leaves the state)
-    if (threadIdx.x == 0) tile_issue_bulk(a, tile, nf, rec_off, b, bar);
+    if (done) {  // uniform across the block (the run stopped: this stage leaves the state)
+        tile_drain(bar, 0);
+        return;
+    }
     if (hx0 >= 0) tile_gather_halo(a, b, nloc, i0, hx0);
     if (hx1 >= 0) tile_gather_halo(a, b, nloc, i1, hx1);
     for (int i = threadIdx.x + 2 * T; i < a.halo_stride; i += T) {
@@ -1163,6 +1202,7 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, int tile, double *
 template <bool EXACT, int MINB>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_release();
     tile_body<EXACT>(a, blockIdx.x, a.partials + blockIdx.x, smem_raw);
 }
 
@@ -1207,10 +1247,13 @@ __device__ __forceinline__ int2 batch_stage_args(const BatchStage &bs, StageArgs
 
 template <bool EXACT, int MINB>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel(BatchStage bs) {
-    if ((int)blockIdx.x >= *bs.n_entries) return;  // uniform across the block
+    pdl_release();
+    if ((int)blockIdx.x >= *bs.n_entries) {  // uniform across the block
+        pdl_wait();
+        return;
+    }
     __shared__ __align__(16) StageArgs sa;
     const int2 e = batch_stage_args(bs, &sa);
-    if (sa.ctl->done) return;  // uniform across the member's blocks
     extern __shared__ __align__(16) unsigned char smem_raw[];
     tile_body<EXACT>(sa, e.y, sa.partials + e.y, smem_raw);
 }

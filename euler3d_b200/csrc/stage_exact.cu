@@ -23,7 +23,7 @@ void launch_update_exact(const StageArgs &a, cudaStream_t s) {
 
 // One stage of every member of a batch: `grid` blocks over the (member, tile) table.
 void launch_batch_exact(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s) {
-    tile_batch_kernel<true, 4><<<grid, kStageThreads, smem_bytes, s>>>(bs);
+    launch_dependent(tile_batch_kernel<true, 4>, grid, kStageThreads, smem_bytes, s, bs);
 }
 
 // The same stage with the warp-specialised persistent kernel: `grid` blocks walk the table.
@@ -40,7 +40,7 @@ void launch_stage_exact(const StageArgs &a, cudaStream_t s, int variant) {
         tile_ws_kernel<WS_EXACT><<<a.pipe_grid, kWsThreads, smem, s>>>(a);
     } else if (variant == 2) {
         const size_t smem = tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
-        tile_kernel<true, 4><<<blocks, kStageThreads, smem, s>>>(a);
+        launch_dependent(tile_kernel<true, 4>, blocks, kStageThreads, smem, s, a);
     } else if (variant == 1) {
         stage_kernel<true, 4><<<blocks, kStageThreads, 0, s>>>(a);
     } else {

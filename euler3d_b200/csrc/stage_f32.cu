@@ -22,7 +22,7 @@ void launch_batch_ws_f32(const BatchStage &bs, int grid, size_t smem_bytes, cuda
 
 // One stage of every member of a batch: `grid` blocks over the (member, tile) table.
 void launch_batch_f32(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s) {
-    tile_batch_kernel_f32<8><<<grid, kStageThreads, smem_bytes, s>>>(bs);
+    launch_dependent(tile_batch_kernel_f32<8>, grid, kStageThreads, smem_bytes, s, bs);
 }
 
 // variant 2: face tiles with registers for four blocks/SM; 3: warp-specialised persistent face
@@ -34,9 +34,9 @@ void launch_stage_f32(const StageArgs &a, cudaStream_t s, int variant) {
         const size_t ws = ws_smem_for(ws_buffer_bytes(WS_F32, a.smem_cells, a.smem_faces, a.max_contrib), a.ws_buffers);
         tile_ws_kernel<WS_F32><<<a.pipe_grid, kWsThreads, ws, s>>>(a);
     } else if (variant == 4) {
-        tile_kernel_f32<8><<<blocks, kStageThreads, smem, s>>>(a);
+        launch_dependent(tile_kernel_f32<8>, blocks, kStageThreads, smem, s, a);
     } else {
-        tile_kernel_f32<4><<<blocks, kStageThreads, smem, s>>>(a);
+        launch_dependent(tile_kernel_f32<4>, blocks, kStageThreads, smem, s, a);
     }
 }
 

@@ -24,7 +24,7 @@ void launch_update_fast(const StageArgs &a, cudaStream_t s) {
 
 // One stage of every member of a batch: `grid` blocks over the (member, tile) table.
 void launch_batch_fast(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s) {
-    tile_batch_kernel<false, 6><<<grid, kStageThreads, smem_bytes, s>>>(bs);
+    launch_dependent(tile_batch_kernel<false, 6>, grid, kStageThreads, smem_bytes, s, bs);
 }
 
 // The same stage with the warp-specialised persistent kernel: `grid` blocks walk the table.
@@ -69,13 +69,13 @@ void launch_stage_fast(const StageArgs &a, cudaStream_t s, int variant) {
     const int blocks = (a.n_cells + kStageThreads - 1) / kStageThreads;
     if (variant == 4) {
         const size_t smem = tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
-        tile_kernel<false, 7><<<blocks, kStageThreads, smem, s>>>(a);
+        launch_dependent(tile_kernel<false, 7>, blocks, kStageThreads, smem, s, a);
     } else if (variant == 3) {
         const size_t smem = ws_smem_for(ws_buffer_bytes(WS_FAST, a.smem_cells, a.smem_faces, a.max_contrib), a.ws_buffers);
         tile_ws_kernel<WS_FAST><<<a.pipe_grid, kWsThreads, smem, s>>>(a);
     } else if (variant == 2) {
         const size_t smem = tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
-        tile_kernel<false, 4><<<blocks, kStageThreads, smem, s>>>(a);
+        launch_dependent(tile_kernel<false, 4>, blocks, kStageThreads, smem, s, a);
     } else if (variant == 1) {
         stage_kernel<false, 5><<<blocks, kStageThreads, 0, s>>>(a);
     } else {

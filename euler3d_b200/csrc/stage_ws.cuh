@@ -91,10 +91,6 @@ __device__ __forceinline__ bool named_sync_or(int id, int threads, bool v) {
     return r != 0;
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // Body of the warp-specialised kernels.  Solo (BATCH false): work item k of the block is tile
 // blockIdx.x + k gridDim.x of the one solver whose arguments `solo` holds.  Batch (BATCH true): work
 // item k is entry blockIdx.x + k gridDim.x of the batch's (member, tile) table; the producer copies
