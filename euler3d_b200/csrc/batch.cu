@@ -65,6 +65,7 @@ struct Batch {
 
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
+    bool graph_apart = false;  // forces_apart() when it was built
     int graph_builds = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
@@ -182,6 +183,15 @@ struct Batch {
 
     bool use_ws() const { return kernel == E3D_BATCH_KERNEL_WS && ws_buffers >= 2; }
 
+    // Force coefficients in a kernel of their own after every iteration: a member's may stop its run, or
+    // the stage kernel has no force blocks.  Otherwise the next first stage integrates them.
+    bool forces_apart() const {
+        if (use_ws()) return true;
+        for (const Member &m : members)
+            if (!m.stopped && !m.last.defer) return true;
+        return false;
+    }
+
     void launch_stage(BatchStage bs) {
         if (use_ws()) {
             bs.ws_buffers = ws_buffers;
@@ -192,19 +202,22 @@ struct Batch {
             else launch_batch_ws_fast(bs, grid, ws_smem, stream);
             return;
         }
-        if (precision == E3D_PREC_FP32_FLUX) launch_batch_f32(bs, tile_cap, smem_cap, stream);
-        else if (precision == E3D_PREC_FP64_EXACT) launch_batch_exact(bs, tile_cap, smem_cap, stream);
-        else launch_batch_fast(bs, tile_cap, smem_cap, stream);
+        const int grid = tile_cap + bs.force_blocks;
+        const size_t smem = with_forces(smem_cap, bs.force_blocks);
+        if (precision == E3D_PREC_FP32_FLUX) launch_batch_f32(bs, grid, smem, stream);
+        else if (precision == E3D_PREC_FP64_EXACT) launch_batch_exact(bs, grid, smem, stream);
+        else launch_batch_fast(bs, grid, smem, stream);
     }
 
     // `iters` iterations (even, so every running member ends on state buffer 0) + the control
     // read-back, as one graph.
-    void build_graph(int iters) {
+    void build_graph(int iters, bool apart) {
         drop_graph();
         const size_t wss = use_ws() ? ws_smem : 0;
-        if (precision == E3D_PREC_FP32_FLUX) prepare_batch_f32(smem_cap, wss);
-        else if (precision == E3D_PREC_FP64_EXACT) prepare_batch_exact(smem_cap, wss);
-        else prepare_batch_fast(smem_cap, wss);
+        const size_t smem = with_forces(smem_cap, 1);
+        if (precision == E3D_PREC_FP32_FLUX) prepare_batch_f32(smem, wss);
+        else if (precision == E3D_PREC_FP64_EXACT) prepare_batch_exact(smem, wss);
+        else prepare_batch_fast(smem, wss);
         static const double alphas[5] = {0.0533, 0.1263, 0.2375, 0.4414, 1.0};
         cudaGraph_t g;
         E3D_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -219,11 +232,17 @@ struct Batch {
                 bs.first_stage = s == 0;
                 bs.last_stage = s == 4;
                 bs.parity = p ^ (s & 1);
+                if (s == 0 && !apart) {
+                    bs.force_blocks = kBatchForceBlocks * member_cap;
+                    bs.n_members = counts.p + 1;
+                    bs.cargs = cargs.p;
+                }
                 launch_stage(bs);
             }
             launch_finalize_batch(fargs.p, counts.p + 1, member_cap, precision == E3D_PREC_FP64_EXACT, stream);
-            launch_coeff_batch(cargs.p, counts.p + 1, 1 - p, member_cap, stream);
+            if (apart) launch_coeff_batch(cargs.p, counts.p + 1, 1 - p, member_cap, stream);
         }
+        if (!apart) launch_coeff_batch(cargs.p, counts.p + 1, 0, member_cap, stream);  // the last iteration's
         launch_control_gather(ctlp.p, counts.p + 1, ctl_all.p, member_cap, stream);
         cudaMemcpyAsync(ctl_host, ctl_all.p, (size_t)member_cap * sizeof(Control), cudaMemcpyDeviceToHost, stream);
         cudaError_t cap = cudaStreamEndCapture(stream, &g);
@@ -232,6 +251,7 @@ struct Batch {
         cudaGraphDestroy(g);
         E3D_CUDA(inst);
         graph_iters = iters;
+        graph_apart = apart;
         graph_builds++;
     }
 
@@ -248,7 +268,8 @@ struct Batch {
         if (running() == 0) return;
         const int every = std::max(2, iters + (iters & 1));
         if (dirty) refresh();
-        if (!graph || graph_iters != every) build_graph(every);
+        const bool apart = forces_apart();
+        if (!graph || graph_iters != every || graph_apart != apart) build_graph(every, apart);
         E3D_CUDA(cudaEventRecord(ev0, stream));
         E3D_CUDA(cudaGraphLaunch(graph, stream));
         E3D_CUDA(cudaEventRecord(ev1, stream));
@@ -256,7 +277,7 @@ struct Batch {
         float ms = 0.f;
         E3D_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
         last_ms = ms;
-        const int64_t step_launches = 7LL * every + 1;
+        const int64_t step_launches = (apart ? 7LL : 6LL) * every + (apart ? 1 : 2);
         launches += step_launches;
         bool halted = false;
         for (size_t k = 0; k < members.size(); k++) {
@@ -377,7 +398,7 @@ e3d_status e3d_batch_add(e3d_batch *batch, e3d_solver *solver, const e3d_run_par
             throw Error(E3D_ERR_INVALID_ARG, "batch members run RK5 without residual smoothing");
         E3D_CUDA(cudaSetDevice(B->device));
         E3D_CUDA(cudaStreamSynchronize(S->stream));  // the solver's own pending work (state uploads)
-        begin_run(S, rp, B->stream);
+        begin_run(S, rp, !forces_decide(rp), B->stream);
         Member m;
         m.S = S;
         std::memcpy(&m.last, S->ctl_host, sizeof(Control));

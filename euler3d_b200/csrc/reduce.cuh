@@ -4,32 +4,13 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "forces.cuh"
 #include "stage.cuh"
 
 namespace e3d {
 
 constexpr int kReduceThreads = 256;   // lanes of the sum of the RMS partials
-constexpr int kCoeffThreads = 512;    // lanes of the force sums
 constexpr int kOrderedThreads = 1024;  // block of FP64_EXACT's RMS kernel
-
-struct CoeffArgs {
-    int n_wall;
-    const int *__restrict__ cell;       // device cell of each wall face, reference wall order
-    const double *__restrict__ svec;    // 3 per wall face: full face normal
-    const double *__restrict__ center;  // 3 per wall face: face centre
-    const double2 *__restrict__ q;
-    const double *__restrict__ w0;      // FP32_FLUX mode: pressure from the double conservative state
-    int w0_stride;
-    double gamma;
-    double p_inf, cp_factor, cref, sref, ref[3];
-    int axis[3], sign[3];
-    Control *ctl;
-    int run_mode;                       // 1: sampled inside e3d_solver_run, apply the stop test
-    int sequential;                     // 1: sum in the reference's wall order (FP64_EXACT)
-    double *__restrict__ out;           // 6 doubles (force, moment) when not in run mode
-    double *__restrict__ cp_out;        // [n_wall] Cp of every wall face (AeroCoefficients::_cp), or null
-    double *__restrict__ samples;       // run mode: 7 doubles (iteration, force, moment) per sample, or null
-};
 
 // Arguments of the RMS / stop-test kernel of one solver.
 struct FinalizeArgs {
@@ -294,48 +275,29 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs &f, Control *ct
         }
     }
     ctl->it += 1;
-    if (ctl->it % ctl->sampling == 0) {
-        ctl->sample_now = 1;
-    } else if (ctl->it >= ctl->max_iter) {
+    const bool sample = ctl->it % ctl->sampling == 0;
+    if (sample) ctl->sample_now = 1;
+    // with a sample pending that may stop the run on its coefficients, its kernel looks at the count
+    if ((!sample || ctl->defer) && ctl->it >= ctl->max_iter) {
         ctl->done = 1;
         ctl->stop_reason = E3D_STOP_MAX_ITER;
     }
 }
 
 // ------------------------------------------------------------------------------ force coefficients
-__device__ __forceinline__ double wall_pressure(const CoeffArgs &a, int c) {
-    if (!a.w0) return __ldcg(&a.q[3 * c + 2].x);
-    const size_t st = (size_t)a.w0_stride;
-    const double rho = __ldcg(a.w0 + c), mu = __ldcg(a.w0 + st + c), mv = __ldcg(a.w0 + 2 * st + c);
-    const double mw = __ldcg(a.w0 + 3 * st + c);
-    return (a.gamma - 1.0) * (__ldcg(a.w0 + 4 * st + c) - 0.5 * (mu * mu + mv * mv + mw * mw) / rho);
-}
-
 // AeroCoefficients::Update (src/solver/AeroCoefficients.cpp:38-52): face terms in parallel; in exact
 // mode each of the six sums by one thread in the reference's wall order, so the sums are the
-// reference's, otherwise by kCoeffThreads lanes; then EulerSolver::ConvergenceCriteria and the CL/CD/CM
-// selection (src/solver/EulerSolver.cpp:132-152, :253-279).  One block of NT threads per solver.
+// reference's, otherwise a fixed-shape tree of kCoeffThreads lanes.  One block of NT threads per solver.
 template <int NT>
 __device__ __forceinline__ void coeff_body(const CoeffArgs &a, Control *ctl, ControlScratch &sh) {
-    if (a.run_mode && (ctl->done || !ctl->sample_now)) return;
+    if (a.run_mode && !forces_due(ctl)) return;
     double (*terms)[kCoeffThreads] = sh.terms;
     if (a.sequential) {
         // the reference's order: one running sum over the wall list, thread k's the k-th
         double acc = 0.0;
         for (int base = 0; base < a.n_wall; base += kCoeffThreads) {
             const int n = min(kCoeffThreads, a.n_wall - base);
-            for (int j = threadIdx.x; j < n; j += NT) {
-                const int i = base + j;
-                double p = wall_pressure(a, a.cell[i]);
-                double cp = a.cp_factor * (p - a.p_inf);
-                if (a.cp_out) a.cp_out[i] = cp;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    double coeff = a.svec[3 * i + k] * cp * a.cref / a.sref;
-                    terms[k][j] = coeff;
-                    terms[3 + k][j] = coeff * a.center[3 * i + k];
-                }
-            }
+            force_terms<NT>(a, base, n, terms);
             __syncthreads();
             if (threadIdx.x < 6)
                 for (int j = 0; j < n; j++) acc += terms[threadIdx.x][j];
@@ -344,38 +306,9 @@ __device__ __forceinline__ void coeff_body(const CoeffArgs &a, Control *ctl, Con
         if (threadIdx.x < 6) terms[threadIdx.x][0] = acc;
         __syncthreads();
     } else {
-        // fixed-shape tree: strided sums of lane t over wall faces t, t + T, t + 2T, ... in that
-        // order (their loads issued four faces at a time), then a pairwise tree (deterministic)
-        constexpr int U = 4;
         for (int lane = threadIdx.x; lane < kCoeffThreads; lane += NT) {
-            double acc[6] = {0, 0, 0, 0, 0, 0};
-            for (int base = lane; base < a.n_wall; base += U * kCoeffThreads) {
-                double p[U], sv[U][3], ce[U][3];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int i = base + u * kCoeffThreads;
-                    if (i < a.n_wall) {
-                        p[u] = wall_pressure(a, a.cell[i]);
-#pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            sv[u][k] = a.svec[3 * i + k];
-                            ce[u][k] = a.center[3 * i + k];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (base + u * kCoeffThreads >= a.n_wall) break;
-                    const double cp = a.cp_factor * (p[u] - a.p_inf);
-                    if (a.cp_out) a.cp_out[base + u * kCoeffThreads] = cp;
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        const double coeff = sv[u][k] * cp * a.cref / a.sref;
-                        acc[k] += coeff;
-                        acc[3 + k] += coeff * ce[u][k];
-                    }
-                }
-            }
+            double acc[6];
+            force_lane(a, lane, acc);
 #pragma unroll
             for (int k = 0; k < 6; k++) terms[k][lane] = acc[k];
         }
@@ -388,48 +321,8 @@ __device__ __forceinline__ void coeff_body(const CoeffArgs &a, Control *ctl, Con
         }
     }
     if (threadIdx.x != 0) return;
-    double F[3], CP[3];
-    for (int k = 0; k < 3; k++) {
-        F[k] = terms[k][0];
-        CP[k] = terms[3 + k][0];
-    }
-    double lever[3] = {a.ref[0] - CP[0], a.ref[1] - CP[1], a.ref[2] - CP[2]};
-    double M[3] = {(F[1] * lever[2] - F[2] * lever[1]) / a.cref, (F[2] * lever[0] - F[0] * lever[2]) / a.cref,
-                   (F[0] * lever[1] - F[1] * lever[0]) / a.cref};
-    if (!a.run_mode) {
-        for (int k = 0; k < 3; k++) {
-            a.out[k] = F[k];
-            a.out[3 + k] = M[k];
-        }
-        return;
-    }
-    double cl = F[a.axis[0]] * a.sign[0], cd = F[a.axis[1]] * a.sign[1], cm = M[a.axis[2]] * a.sign[2];
-    double tol = ctl->min_aero;
-    bool ok = fabs(ctl->cl - cl) < tol && fabs(ctl->cd - cd) < tol && fabs(ctl->cm - cm) < tol;
-    ctl->counter = ok ? ctl->counter + 1 : 0;
-    if (a.samples && ctl->n_samples < ctl->sample_cap) {  // a residuals.dat row (EulerSolver::PrintInfo)
-        double *s = a.samples + 7 * (size_t)ctl->n_samples;
-        s[0] = ctl->it;
-        for (int k = 0; k < 3; k++) {
-            s[1 + k] = F[k];
-            s[4 + k] = M[k];
-        }
-    }
-    ctl->n_samples += 1;
-    ctl->cl = cl;
-    ctl->cd = cd;
-    ctl->cm = cm;
-    for (int k = 0; k < 3; k++) {
-        ctl->force[k] = F[k];
-        ctl->moment[k] = M[k];
-    }
-    if (ctl->counter >= 2) {
-        ctl->done = 1;
-        ctl->stop_reason = E3D_STOP_COEFFICIENTS;
-    } else if (ctl->it >= ctl->max_iter) {
-        ctl->done = 1;
-        ctl->stop_reason = E3D_STOP_MAX_ITER;
-    }
+    const double F[3] = {terms[0][0], terms[1][0], terms[2][0]}, CP[3] = {terms[3][0], terms[4][0], terms[5][0]};
+    force_finish(a, ctl, F, CP);
 }
 
 }  // namespace e3d

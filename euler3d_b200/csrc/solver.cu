@@ -856,7 +856,8 @@ static void create_solver(const e3d_mesh_desc *d, const e3d_flow_params *p, Solv
     S->n_blocks = (N + kStageThreads - 1) / kStageThreads;
     S->partials.alloc(S->n_blocks);
     S->staging.alloc(8 * (size_t)S->state_size());
-    S->scratch.alloc(6);
+    S->scratch.alloc(6 + 1 + 6 * (size_t)d->n_wall);  // coefficients; force blocks' arrival count and terms
+    E3D_CUDA(cudaMemsetAsync(S->scratch.p, 0, S->scratch.n * sizeof(double), s));
     E3D_CUDA(cudaMalloc(&S->ctl, sizeof(Control)));
     E3D_CUDA(cudaHostAlloc(&S->ctl_host, sizeof(Control), cudaHostAllocDefault));
     E3D_CUDA(cudaMemsetAsync(S->ctl, 0, sizeof(Control), s));
@@ -918,7 +919,7 @@ static Solver *solo(e3d_solver *s) {
 // A fresh control block for a run -- a new EulerSolver's counters (_nbInteration = 0,
 // _CL = _CD = _CM = 0, src/solver/EulerSolver.cpp:21-58) -- keeping whether the loaded interior
 // Mach still holds.  Reads the old block back first (synchronises stream s once).
-static void init_control(Solver *S, const e3d_run_params *rp, int max_iter, int hist_cap, int sample_cap,
+static void init_control(Solver *S, const e3d_run_params *rp, int max_iter, int hist_cap, int sample_cap, bool defer,
                          cudaStream_t s) {
     E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
     E3D_CUDA(cudaStreamSynchronize(s));
@@ -934,6 +935,7 @@ static void init_control(Solver *S, const e3d_run_params *rp, int max_iter, int 
     init.stall_window = std::max(rp->stall_window, 0);
     init.stall_below = rp->stall_below;
     init.done = max_iter == 0;
+    init.defer = defer;
     std::memcpy(S->ctl_host, &init, sizeof init);
     E3D_CUDA(cudaMemcpyAsync(S->ctl, S->ctl_host, sizeof(Control), cudaMemcpyHostToDevice, s));
 }
@@ -950,7 +952,7 @@ static void state_to_buffer0(Solver *S, cudaStream_t s) {
     S->cur = 0;
 }
 
-void begin_run(Solver *S, const e3d_run_params *rp, cudaStream_t s) {
+void begin_run(Solver *S, const e3d_run_params *rp, bool defer, cudaStream_t s) {
     if (rp->sampling <= 0) throw Error(E3D_ERR_INVALID_ARG, "sampling must be a positive integer");
     if (!(rp->min_residual_drop >= 0.0)) throw Error(E3D_ERR_INVALID_ARG, "min_residual_drop must be >= 0");
     const int max_iter = std::max(rp->max_iter, 0);
@@ -986,7 +988,7 @@ void begin_run(Solver *S, const e3d_run_params *rp, cudaStream_t s) {
     }
     // a fresh AeroCoefficients: Cp of every wall face zero until the first sample
     if (S->n_wall) E3D_CUDA(cudaMemsetAsync(S->wall_cp.p, 0, S->n_wall * sizeof(double), s));
-    init_control(S, rp, max_iter, S->hist_cap, S->sample_cap, s);
+    init_control(S, rp, max_iter, S->hist_cap, S->sample_cap, defer, s);
     state_to_buffer0(S, s);
     S->records_valid = true;
 }
@@ -1146,9 +1148,9 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
         Solver *S = solo(solver);
         E3D_CUDA(cudaSetDevice(S->device));
         if (rp->sampling <= 0) throw Error(E3D_ERR_INVALID_ARG, "sampling must be a positive integer");
+        if (!(rp->min_residual_drop >= 0.0)) throw Error(E3D_ERR_INVALID_ARG, "min_residual_drop must be >= 0");
         e3d_run_stats st{};
         const int max_iter = std::max(rp->max_iter, 0);
-        begin_run(S, rp, S->stream);
         if (rp->stage_kernel > 0) {
             const int v = rp->stage_kernel - 1;
             if (!S->variant_ok(v))
@@ -1174,6 +1176,10 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
         std::unique_lock<std::mutex> resident;
         if (rp->profile_stages == 0 && !S->variant_forced && S->device < 64 && S->resident_ready())
             resident = std::unique_lock<std::mutex>(resident_busy[S->device], std::try_to_lock);
+        // Forces that cannot stop the run are left to the next iteration's first stage (the resident
+        // kernel's control block has its own way, and timed stages hold nothing else).
+        const bool defer = !resident.owns_lock() && rp->profile_stages == 0 && S->can_defer() && !forces_decide(rp);
+        begin_run(S, rp, defer, S->stream);
         if (resident.owns_lock()) {
             // every tile resident: whole iterations in one launch.  The host looks at the stop flag as
             // often as the caller asks, otherwise every kResidentIterations (a launch costs less than
@@ -1195,7 +1201,7 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
             int every = rp->check_every > 0 ? rp->check_every : 32;
             every += every & 1;  // whole graphs start and end on buffer 0
             const bool timed = rp->profile_stages == 2;
-            if (timed || max_iter >= every) S->build_graph(every, timed);
+            if (timed || max_iter >= every) S->build_graph(every, timed, defer);
             E3D_CUDA(cudaEventRecord(S->ev0, S->stream));
             int launched_iters = 0;
             int n_before = 0;  // iterations done before this graph launch (the control block's RMS count)
@@ -1209,10 +1215,11 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
                 if (n == every) {
                     E3D_CUDA(cudaGraphLaunch(S->graph, S->stream));
                 } else {
-                    for (int i = 0; i < n; i++) S->enqueue_iteration(i & 1);
+                    for (int i = 0; i < n; i++) S->enqueue_iteration(i & 1, nullptr, defer);
+                    if (defer) S->enqueue_forces(n & 1);
                     E3D_CUDA(cudaGetLastError());
                 }
-                launches += (int64_t)S->kernels_per_iteration() * n;
+                launches += (int64_t)S->kernels_per_iteration(defer) * n + (defer ? 1 : 0);
                 launched_iters += n;
                 E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, S->stream));
                 E3D_CUDA(cudaStreamSynchronize(S->stream));
@@ -1338,7 +1345,7 @@ e3d_status e3d_solver_run_noalloc(e3d_solver *solver, const e3d_run_params *rp, 
         E3D_CUDA(cudaMemsetAsync(hist, 0, (size_t)std::max(max_iter, 1) * sizeof(double), S->stream));
         // a fresh AeroCoefficients, as e3d_solver_run starts one: wall Cp zero until the first sample
         if (S->n_wall) E3D_CUDA(cudaMemsetAsync(S->wall_cp.p, 0, S->n_wall * sizeof(double), S->stream));
-        init_control(S, rp, max_iter, kNoAllocMaxIter, 0, S->stream);
+        init_control(S, rp, max_iter, kNoAllocMaxIter, 0, false, S->stream);
         state_to_buffer0(S, S->stream);
         // the handle's RMS history and sample record still hold an earlier run's: this run keeps
         // neither there (its RMS history goes to rms_history), so the queries of them report none

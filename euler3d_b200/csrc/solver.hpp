@@ -15,11 +15,11 @@
 
 namespace e3d {
 
-void launch_stage_exact(const StageArgs &a, cudaStream_t s, int variant);
-void launch_stage_fast(const StageArgs &a, cudaStream_t s, int variant);
+void launch_stage_exact(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant);
+void launch_stage_fast(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant);
 void prepare_tile_exact(size_t smem_bytes, size_t pipe_smem_bytes);
 void prepare_tile_fast(size_t smem_bytes, size_t pipe_smem_bytes);
-void launch_stage_f32(const StageArgs &a, cudaStream_t s, int variant);
+void launch_stage_f32(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant);
 void prepare_tile_f32(size_t smem_bytes, size_t ws_smem_bytes);
 // gather (two register budgets), face tiles, warp-specialised persistent face tiles, face tiles at 7 blocks/SM,
 // face colouring at 128 and at 512 faces per block
@@ -151,6 +151,7 @@ struct Solver {
 
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
+    bool graph_defer = false;             // its forces are deferred to the next iteration's first stage
     bool graph_timed = false;             // the graph records graph_ev around its stage kernels
     std::vector<cudaEvent_t> graph_ev;    // [iteration][stage][begin, end] of a timed graph
     Batch *batch = nullptr;        // the batch running this solver, if any (batch.cu)
@@ -375,7 +376,7 @@ struct Solver {
     // The launches of one stage with variant v (face colouring: one per class and the update).
     int stage_launches(int v) const { return v >= kColourVariant ? n_colours + 1 : 1; }
 
-    void launch_stage(const StageArgs &a, int v = -1) {
+    void launch_stage(const StageArgs &a, int v = -1, const CoeffArgs &c = {}) {
         if (v < 0) v = variant;
         if (v >= kColourVariant) {  // the accumulator is cleared, every class adds, the update reads it
             E3D_CUDA(cudaMemsetAsync(colour_r.p, 0, colour_r.n * sizeof(double2), stream));
@@ -386,9 +387,9 @@ struct Solver {
             launch_colour_finish_fast(a, colour_r.p, stream);
             return;
         }
-        if (f32) launch_stage_f32(a, stream, v);
-        else if (prm.precision == E3D_PREC_FP64_EXACT) launch_stage_exact(a, stream, v);
-        else launch_stage_fast(a, stream, v);
+        if (f32) launch_stage_f32(a, c, stream, v);
+        else if (prm.precision == E3D_PREC_FP64_EXACT) launch_stage_exact(a, c, stream, v);
+        else launch_stage_fast(a, c, stream, v);
     }
 
     // Time every stage-kernel variant on this mesh and keep the fastest.  The trial launches
@@ -477,6 +478,8 @@ struct Solver {
         c.out = out;
         c.cp_out = wall_cp.p;
         c.samples = run_mode ? samples.p : nullptr;
+        c.arrivals = reinterpret_cast<unsigned *>(scratch.p + 6);
+        c.terms = scratch.p + 7;
         return c;
     }
 
@@ -488,19 +491,27 @@ struct Solver {
     // Stages per iteration (RK5: 5; explicit Euler: 1) and kernels per stage and per iteration.
     int n_stages() const { return euler() ? 1 : 5; }
     int kernels_per_stage() const { return stage_launches(variant) + (smoothing ? 3 : 0); }
-    int kernels_per_iteration() const { return n_stages() * kernels_per_stage() + 2; }
+    int kernels_per_iteration(bool defer = false) const { return n_stages() * kernels_per_stage() + (defer ? 1 : 2); }
+
+    // Can the first stage integrate the forces (force_block)?  The face-tile kernels do.
+    bool can_defer() const { return variant == 2 || variant == 4; }
 
     // Stage s of an iteration from q[b] (EulerSolver::RungeKutta, src/solver/EulerSolver.cpp:425-472,
     // or EulerSolver::EulerExplicit, :419-423).  Without smoothing one fused kernel; with it the
     // residual phase writes R, two Jacobi passes smooth it (EulerSolver::smoothResiduals, :483-518,
     // called by Run() :91-93 for the first stage and by RungeKutta :456-458 for the others) and the
     // update kernel applies it.
-    void enqueue_stage(int b, int s, double *part) {
+    void enqueue_stage(int b, int s, double *part, bool defer = false) {
         static const double alphas[5] = {0.0533, 0.1263, 0.2375, 0.4414, 1.0};
         StageArgs a = stage_args(b, euler() ? 1.0 : alphas[s], s == 0, euler() || s == 4);
         a.partials = part;
+        CoeffArgs c{};
+        if (defer && s == 0) {
+            a.force_blocks = std::max(1, std::min(kMaxForceBlocks, (n_wall + kForceThreads - 1) / kForceThreads));
+            c = coeff_args(b, 1, nullptr);
+        }
         if (!smoothing) {
-            launch_stage(a);
+            launch_stage(a, -1, c);
             return;
         }
         const size_t n5 = 5 * (size_t)w0_stride;
@@ -510,7 +521,7 @@ struct Solver {
         ar.ghost_out = a.last_stage;  // the residual phase of the last stage leaves the ghosts
         ar.last_stage = 0;
         ar.r_dev = r0;
-        launch_stage(ar);
+        launch_stage(ar, -1, c);
         E3D_CUDA(cudaMemsetAsync(smooth_flags.p, 0, 2 * sizeof(unsigned long long), stream));
         SmoothArgs sa{N, w0_stride, nb_ptr.p, nb.p, den.p, r0, r0, r1, smooth_flags.p, ctl, 0};
         launch_smooth(sa, stream);
@@ -526,23 +537,28 @@ struct Solver {
     // One iteration of EulerSolver::Run (src/solver/EulerSolver.cpp:84-153) starting from q[in_buf];
     // returns the kernels launched.  With ev, event pair ev[2 s], ev[2 s + 1] brackets stage s (as
     // external event-record nodes when the stream is being captured).
-    int enqueue_iteration(int in_buf, const cudaEvent_t *ev = nullptr) {
+    // With `defer` the forces of an iteration are the next one's first stage's (Control::defer), and the
+    // caller ends the sequence with enqueue_forces.
+    int enqueue_iteration(int in_buf, const cudaEvent_t *ev = nullptr, bool defer = false) {
         int b = in_buf;
         for (int s = 0; s < n_stages(); s++) {
             if (ev) E3D_CUDA(cudaEventRecordWithFlags(ev[2 * s], stream, cudaEventRecordExternal));
-            enqueue_stage(b, s, partials.p);
+            enqueue_stage(b, s, partials.p, defer);
             if (ev) E3D_CUDA(cudaEventRecordWithFlags(ev[2 * s + 1], stream, cudaEventRecordExternal));
             b = 1 - b;
         }
         launch_finalize(finalize_args(partials.p, hist.p), stream);
-        launch_coeff(coeff_args(b, 1, nullptr), stream);
-        return kernels_per_iteration();
+        if (!defer) enqueue_forces(b);
+        return kernels_per_iteration(defer);
     }
+
+    // The force coefficients that are due of the state in buffer b.
+    void enqueue_forces(int b) { launch_coeff(coeff_args(b, 1, nullptr), stream); }
 
     // A graph of `iters` iterations; with `timed`, an event pair around every stage kernel (see
     // e3d_run_params.profile_stages = 2).
-    void build_graph(int iters, bool timed = false) {
-        if (graph && graph_iters == iters && graph_timed == timed) return;
+    void build_graph(int iters, bool timed, bool defer) {
+        if (graph && graph_iters == iters && graph_timed == timed && graph_defer == defer) return;
         if (graph) {
             cudaGraphExecDestroy(graph);
             graph = nullptr;
@@ -557,9 +573,10 @@ struct Solver {
         E3D_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         int b = 0;
         for (int i = 0; i < iters; i++) {
-            enqueue_iteration(b, timed ? graph_ev.data() + 2 * (size_t)n_stages() * i : nullptr);
+            enqueue_iteration(b, timed ? graph_ev.data() + 2 * (size_t)n_stages() * i : nullptr, defer);
             b = 1 - b;  // five stages flip the buffer once per iteration
         }
+        if (defer) enqueue_forces(b);
         cudaError_t cap = cudaStreamEndCapture(stream, &g);
         E3D_CUDA(cap);
         cudaError_t inst = cudaGraphInstantiate(&graph, g, 0);
@@ -567,6 +584,7 @@ struct Solver {
         E3D_CUDA(inst);
         graph_iters = iters;
         graph_timed = timed;
+        graph_defer = defer;
     }
 };
 
@@ -574,7 +592,10 @@ inline Solver *as_solver(e3d_solver *s) { return reinterpret_cast<Solver *>(s); 
 
 // Start of a run (e3d_solver_run and e3d_batch_add): history capacity, a fresh control block
 // and the current state moved to buffer 0, all enqueued on stream s.
-void begin_run(Solver *S, const e3d_run_params *rp, cudaStream_t s);
+// defer: force coefficients that cannot stop the run are left to the next iteration's first stage.
+void begin_run(Solver *S, const e3d_run_params *rp, bool defer, cudaStream_t s);
+// Can the force coefficients stop a run (the coefficient test is on)?
+inline bool forces_decide(const e3d_run_params *rp) { return rp->min_aerocoeff_error > 0.0; }
 // Run statistics from a control block read back from the device.
 void stats_from_control(const Control &c, e3d_run_stats *st);
 // Take a solver out of the batch that holds it (e3d_solver_destroy of a member).

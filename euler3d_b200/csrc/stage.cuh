@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "euler3d_b200.h"
+#include "forces.cuh"
 
 namespace e3d {
 
@@ -39,31 +40,7 @@ struct Freestream {
     double rho, u, v, w, p, E, H, M;
 };
 
-// Run control shared by the kernels of e3d_solver_run; lives in device memory.
-struct Control {
-    int done;          // nonzero: every later kernel returns at once
-    int stop_reason;   // E3D_STOP_*
-    int it;            // EulerSolver::_nbInteration
-    int n_rms;         // iterations whose RMS has been computed
-    int counter;       // consecutive stagnated coefficient samples (src/solver/EulerSolver.cpp:142-147)
-    int sample_now;    // this iteration samples the force coefficients
-    int minit_valid;   // interior Mach of the loaded state still holds (no stage has run since)
-    int nonfinite;     // the RMS became NaN/Inf
-    int max_iter, sampling, hist_cap;
-    int fault;         // a bounded wait in a kernel gave up
-    double min_res, min_aero, last_rms, cl, cd, cm;
-    double min_drop;   // > 0: also stop once the RMS is below min_drop x the run's first RMS
-    double rms0;       // RMS of the run's first iteration
-    int n_samples;     // coefficient samples taken (residuals.dat rows)
-    int sample_cap;    // capacity of the sample record
-    int stall_window;  // > 0: stop once the RMS has set no new minimum for this many iterations
-    int since_best;    // iterations since the RMS last set a new minimum
-    double best_rms;   // smallest RMS of the run so far
-    double stall_below;  // the stall test counts only once RMS < stall_below x the first RMS (0: always)
-    double force[3], moment[3];
-};
-
-struct StageArgs {
+struct alignas(16) StageArgs {  // bulk-copied by tile_ws_batch_kernel
     int n_cells, n_ghosts;
     const int *__restrict__ cptr;
     const int2 *__restrict__ cf;
@@ -101,7 +78,7 @@ struct StageArgs {
     int *fault;                      // set when a bounded wait gives up (reported as a timeout)
     int halo_stride;                 // entries per tile in tile_halo (the largest halo)
     int n_tiles;                     // tiles of the mesh
-    int pipe_grid;                   // tile_ws_kernel: persistent blocks (one per SM)
+    int pipe_grid;                   // the GPU's SMs, or the tiles if fewer (tile_ws_kernel's blocks)
     int ws_buffers;                  // tile_ws_kernel: tile buffers in shared memory
     // FP32_FLUX mode: float cell records (rho,u,v,w | p,H,sqrt(rho),rsqrt(gamma p rho)), float
     // face records and float cell geometry; W0 stays double
@@ -118,6 +95,8 @@ struct StageArgs {
                                      // summed sequentially like EulerSolver::computeRMS; else null
     int wait_polls;                  // polls of a tile's data barrier before the wait gives up (kWaitLimit;
                                      // fewer, down to 0, only to exercise the timeout path)
+    int force_blocks;                // blocks at the front of the grid for the deferred forces (in an
+                                     // iteration's first stage, else 0)
     int ghost_out;                   // write wall / symmetry ghost records although this is not a last
                                      // stage (the residual phase of a split last stage)
 };
@@ -997,17 +976,12 @@ __device__ __forceinline__ TileBuf tile_buf_at(unsigned char *base, int LC, int 
 __device__ __forceinline__ void tile_issue_mesh(const StageArgs &a, int tile, int nf, long long rec_off,
                                                 const TileBuf &b, uint64_t *bar) {
     const int T = kTileCells, MC = a.max_contrib;
-    const int c0 = tile * T, nloc = min(T, a.n_cells - c0);
     const uint32_t b_rec = round16(40u * (uint32_t)nf);
-    const uint32_t b_w0 = round16((uint32_t)nloc * 8u);  // stays inside the padded rows
-    const uint32_t b_cg = (uint32_t)nloc * 32u;
     const uint32_t b_ct = (uint32_t)MC * T * 2u;
     mbar_expect_tx(bar, b_rec + b_ct);
     const uint64_t once = l2_evict_first();
     bulk_g2s_hint(b.rec, a.tile_rec + rec_off, b_rec, bar, once);
     bulk_g2s_hint(b.ct, a.tile_contrib + (size_t)tile * MC * T, b_ct, bar, once);
-    for (int k = 0; k < 5; k++) bulk_prefetch_l2(a.w0 + (size_t)k * a.w0_stride + c0, b_w0);
-    bulk_prefetch_l2(a.cgeo + c0, b_cg);
 }
 
 __device__ __forceinline__ void tile_issue_state(const StageArgs &a, int tile, const TileBuf &b, uint64_t *bar) {
@@ -1016,6 +990,19 @@ __device__ __forceinline__ void tile_issue_state(const StageArgs &a, int tile, c
     mbar_expect_tx(bar, b_state);
     bulk_g2s(b.st, a.qin + 3 * (size_t)c0, b_state, bar);
 }
+
+// L2 prefetches of what the update will read from global memory: W0 rows and cell geometry.
+__device__ __forceinline__ void tile_prefetch(const StageArgs &a, int tile, const void *geo, uint32_t geo_bytes) {
+    const int c0 = tile * kTileCells;
+    const uint32_t nloc = (uint32_t)min(kTileCells, a.n_cells - c0);
+    for (int k = 0; k < 5; k++) bulk_prefetch_l2(a.w0 + (size_t)k * a.w0_stride + c0, round16(nloc * 8u));  // padded rows
+    bulk_prefetch_l2(static_cast<const char *>(geo) + (size_t)geo_bytes * c0, nloc * geo_bytes);
+}
+
+// Blocks that may start while the previous kernel runs: they copy the mesh's data before they wait for
+// it.  Later blocks find it done and copy the states first, which the flux phase needs first (issuing
+// them after the records and prefetches cost the FP32_FLUX stage 3 %).
+__device__ __forceinline__ bool early_block(const StageArgs &a) { return (int)blockIdx.x < 8 * a.pipe_grid; }
 
 // Halo state i of the tile (global cell h) into st[nloc + i] with three 16-byte cp.async.
 __device__ __forceinline__ void tile_gather_halo(const StageArgs &a, const TileBuf &b, int nloc, int i, int h) {
@@ -1129,7 +1116,8 @@ __device__ __forceinline__ void tile_drain(uint64_t *bar, uint32_t parity) {
 }
 
 // Had the run stopped when the block started?  Before pdl_wait the kernel that stops a run may still be
-// running, so only "yes" is final (the flag is cleared by the host alone).
+// running, so only "yes" is final (the flag is cleared by the host alone): it saves the block's loads,
+// and the flag read after the wait decides.
 __device__ __forceinline__ bool run_stopped(const StageArgs &a) {
     return !a.residual_only && *(volatile const int *)&a.ctl->done;
 }
@@ -1158,35 +1146,40 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, int tile, double *
     const int hx1 = i1 < a.halo_stride ? hrow[i1] : -1;
     const int fp0 = a.tile_face_ptr[tile], fp1 = a.tile_face_ptr[tile + 1];
     const long long rec_off = a.tile_rec_off[tile];
+    const bool stopped = run_stopped(a), early = early_block(a);
     const int nf = fp1 - fp0;
 
     if (threadIdx.x == 0) {
         mbar_init(bar, 2);
-        if (run_stopped(a)) mbar_arrive(bar);
-        else tile_issue_mesh(a, tile, nf, rec_off, b, bar);
+        if (early && !stopped) tile_issue_mesh(a, tile, nf, rec_off, b, bar);
     }
     pdl_wait();
-    const bool done = !a.residual_only && a.ctl->done;
+    const bool done = !a.residual_only && a.ctl->done;  // looked at after the copies have landed
     if (threadIdx.x == 0) {
-        if (done) mbar_arrive(bar);
-        else tile_issue_state(a, tile, b, bar);
+        if (stopped) {
+            mbar_arrive(bar);
+            mbar_arrive(bar);
+        } else {
+            tile_issue_state(a, tile, b, bar);
+            if (!early) tile_issue_mesh(a, tile, nf, rec_off, b, bar);
+            tile_prefetch(a, tile, a.cgeo, 32u);
+        }
     }
-    __syncthreads();
-    if (done) {  // uniform across the block (the run stopped: this stage leaves the state)
-        tile_drain(bar, 0);
-        return;
-    }
-    if (hx0 >= 0) tile_gather_halo(a, b, nloc, i0, hx0);
-    if (hx1 >= 0) tile_gather_halo(a, b, nloc, i1, hx1);
-    for (int i = threadIdx.x + 2 * T; i < a.halo_stride; i += T) {
-        const int h = hrow[i];
-        if (h >= 0) tile_gather_halo(a, b, nloc, i, h);
+    if (!stopped) {
+        if (hx0 >= 0) tile_gather_halo(a, b, nloc, i0, hx0);
+        if (hx1 >= 0) tile_gather_halo(a, b, nloc, i1, hx1);
+        for (int i = threadIdx.x + 2 * T; i < a.halo_stride; i += T) {
+            const int h = hrow[i];
+            if (h >= 0) tile_gather_halo(a, b, nloc, i, h);
+        }
     }
     cp_async_wait_all();
+    __syncthreads();  // the barrier is initialised
     if (!tile_wait(a, bar, 0)) {
         tile_drain(bar, 0);
         return;
     }
+    if (done) return;  // uniform across the block (the run stopped: this stage leaves the state)
     const ArgStep sp{a};
     tile_fluxes<EXACT, kStageThreads>(a, sp, b, fs, threadIdx.x, nf, c0);
     double W0[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1200,10 +1193,16 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, int tile, double *
 }
 
 template <bool EXACT, int MINB>
-__global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel(StageArgs a) {
+__global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel(StageArgs a, const __grid_constant__ CoeffArgs c) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     pdl_release();
-    tile_body<EXACT>(a, blockIdx.x, a.partials + blockIdx.x, smem_raw);
+    const int tile = (int)blockIdx.x - a.force_blocks;
+    if (tile < 0) {
+        pdl_wait();
+        force_block(c, blockIdx.x, a.force_blocks, smem_raw);
+        return;
+    }
+    tile_body<EXACT>(a, tile, a.partials + tile, smem_raw);
 }
 
 // ---- several solvers ("members") in one grid
@@ -1216,6 +1215,10 @@ struct BatchStage {
     const StageArgs *__restrict__ args;  // member m reading state buffer b: args[2 * m + b]
     const int2 *__restrict__ table;      // block -> (member, tile of that member)
     const int *__restrict__ n_entries;   // valid table entries; later blocks return at once
+    // deferred forces (an iteration's first stage): kBatchForceBlocks blocks per member at the front of the grid
+    int force_blocks;
+    const int *__restrict__ n_members;
+    const CoeffArgs *__restrict__ cargs; // member m, state buffer b: cargs[2 * m + b]
     double alpha;
     int first_stage, last_stage, parity;
     int ws_buffers, ws_stride;           // tile_ws_batch_kernel: buffers, bytes per buffer
@@ -1224,8 +1227,8 @@ static_assert(sizeof(StageArgs) % 4 == 0, "StageArgs is copied in 4-byte words")
 
 // The block's member arguments into shared memory, with the stage's own alpha and flags written in
 // place of the member's as the words are copied (one barrier).
-__device__ __forceinline__ int2 batch_stage_args(const BatchStage &bs, StageArgs *sa) {
-    const int2 e = bs.table[blockIdx.x];
+__device__ __forceinline__ int2 batch_stage_args(const BatchStage &bs, int entry, StageArgs *sa) {
+    const int2 e = bs.table[entry];
     const uint32_t *src = reinterpret_cast<const uint32_t *>(bs.args + 2 * e.x + bs.parity);
     uint32_t *dst = reinterpret_cast<uint32_t *>(sa);
     constexpr int kAlpha = (int)(offsetof(StageArgs, alpha) / 4), kFirst = (int)(offsetof(StageArgs, first_stage) / 4);
@@ -1245,16 +1248,28 @@ __device__ __forceinline__ int2 batch_stage_args(const BatchStage &bs, StageArgs
     return e;
 }
 
+// The table entry of a batch stage's block; -1 for a block that has none and is done: one of the
+// deferred forces' (its member's forces integrated), or one past the table.
+__device__ __forceinline__ int batch_entry(const BatchStage &bs, unsigned char *smem_raw) {
+    const int entry = (int)blockIdx.x - bs.force_blocks;
+    if (entry >= 0 && entry < *bs.n_entries) return entry;
+    pdl_wait();
+    if (entry < 0) {
+        const int m = (int)blockIdx.x / kBatchForceBlocks;
+        if (m < *bs.n_members)
+            force_block(bs.cargs[2 * m + bs.parity], (int)blockIdx.x % kBatchForceBlocks, kBatchForceBlocks, smem_raw);
+    }
+    return -1;
+}
+
 template <bool EXACT, int MINB>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel(BatchStage bs) {
-    pdl_release();
-    if ((int)blockIdx.x >= *bs.n_entries) {  // uniform across the block
-        pdl_wait();
-        return;
-    }
-    __shared__ __align__(16) StageArgs sa;
-    const int2 e = batch_stage_args(bs, &sa);
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_release();
+    const int entry = batch_entry(bs, smem_raw);
+    if (entry < 0) return;  // uniform across the block
+    __shared__ __align__(16) StageArgs sa;
+    const int2 e = batch_stage_args(bs, entry, &sa);
     tile_body<EXACT>(sa, e.y, sa.partials + e.y, smem_raw);
 }
 
@@ -1281,6 +1296,11 @@ __global__ void __launch_bounds__(kStageThreads) update_kernel(StageArgs a) {
         r2 = finish_cell<EXACT>(a, ArgStep{a}, c, me, r_me, R, W0, a.cgeo[c], out);
     }
     if (a.last_stage) block_sum_store(r2, a.partials + blockIdx.x);
+}
+
+// Dynamic shared memory a stage kernel is launched with: the force blocks at its front need their own.
+inline size_t with_forces(size_t smem, int force_blocks) {
+    return force_blocks && smem < kForceSmem ? kForceSmem : smem;
 }
 
 // Dynamic shared memory of tile_kernel.

@@ -7,7 +7,7 @@ namespace e3d {
 
 // Dynamic shared memory the tile kernels may use (raised before their first launch).
 void prepare_tile_exact(size_t smem_bytes, size_t pipe_smem_bytes) {
-    raise_smem_limit((const void *)tile_kernel<true, 4>, smem_bytes);
+    raise_smem_limit((const void *)tile_kernel<true, 4>, with_forces(smem_bytes, 1));
     if (pipe_smem_bytes) raise_smem_limit((const void *)tile_ws_kernel<WS_EXACT>, pipe_smem_bytes);
 }
 
@@ -33,14 +33,14 @@ void launch_batch_ws_exact(const BatchStage &bs, int grid, size_t smem_bytes, cu
 
 // variant 0: gather kernel, registers for 2 blocks/SM; 1: gather kernel, 4 blocks/SM;
 // 2: face tiles, one block per tile (4 blocks/SM); 3: face tiles, persistent and warp-specialised
-void launch_stage_exact(const StageArgs &a, cudaStream_t s, int variant) {
+void launch_stage_exact(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant) {
     const int blocks = (a.n_cells + kStageThreads - 1) / kStageThreads;
     if (variant == 3) {
         const size_t smem = ws_smem_for(ws_buffer_bytes(WS_EXACT, a.smem_cells, a.smem_faces, a.max_contrib), a.ws_buffers);
         tile_ws_kernel<WS_EXACT><<<a.pipe_grid, kWsThreads, smem, s>>>(a);
     } else if (variant == 2) {
         const size_t smem = tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
-        launch_dependent(tile_kernel<true, 4>, blocks, kStageThreads, smem, s, a);
+        launch_dependent(tile_kernel<true, 4>, blocks + a.force_blocks, kStageThreads, with_forces(smem, a.force_blocks), s, a, c);
     } else if (variant == 1) {
         stage_kernel<true, 4><<<blocks, kStageThreads, 0, s>>>(a);
     } else {

@@ -262,55 +262,52 @@ __device__ __forceinline__ void tile_body_f32(const StageArgs &a, int tile, doub
     const int hx1 = i1 < a.halo_stride ? hrow[i1] : -1;
     const int fp0 = a.tile_face_ptr[tile], fp1 = a.tile_face_ptr[tile + 1];
     const long long rec_off = a.tile_rec32_off[tile];
+    const bool stopped = run_stopped(a), early = early_block(a);
     const int nf = fp1 - fp0;
 
+    auto issue_mesh = [&] {
+        const uint32_t b_rec = round16(24u * (uint32_t)nf), b_ct = (uint32_t)MC * T * 2u;
+        mbar_expect_tx(bar, b_rec + b_ct);
+        const uint64_t once = l2_evict_first();
+        bulk_g2s_hint(b.rec, a.tile_rec32 + rec_off, b_rec, bar, once);
+        bulk_g2s_hint(b.ct, a.tile_contrib + (size_t)tile * MC * T, b_ct, bar, once);
+    };
     if (threadIdx.x == 0) {
         mbar_init(bar, 2);
-        if (run_stopped(a)) {
-            mbar_arrive(bar);
-        } else {
-            const uint32_t b_rec = round16(24u * (uint32_t)nf);
-            const uint32_t b_w0 = round16((uint32_t)nloc * 8u);
-            const uint32_t b_cg = (uint32_t)nloc * 16u;
-            const uint32_t b_ct = (uint32_t)MC * T * 2u;
-            mbar_expect_tx(bar, b_rec + b_ct);
-            const uint64_t once = l2_evict_first();
-            bulk_g2s_hint(b.rec, a.tile_rec32 + rec_off, b_rec, bar, once);
-            bulk_g2s_hint(b.ct, a.tile_contrib + (size_t)tile * MC * T, b_ct, bar, once);
-            for (int k = 0; k < 5; k++) bulk_prefetch_l2(a.w0 + (size_t)k * a.w0_stride + c0, b_w0);
-            bulk_prefetch_l2(a.cgeo32 + c0, b_cg);
-        }
+        if (early && !stopped) issue_mesh();
     }
     pdl_wait();
-    const bool done = !a.residual_only && a.ctl->done;
+    const bool done = !a.residual_only && a.ctl->done;  // looked at after the copies have landed
     if (threadIdx.x == 0) {
-        if (done) {
+        if (stopped) {
+            mbar_arrive(bar);
             mbar_arrive(bar);
         } else {
             mbar_expect_tx(bar, (uint32_t)nloc * 32u);
             bulk_g2s(b.st, a.q32in + 2 * (size_t)c0, (uint32_t)nloc * 32u, bar);
+            if (!early) issue_mesh();
+            tile_prefetch(a, tile, a.cgeo32, 16u);
         }
-    }
-    __syncthreads();
-    if (done) {  // uniform across the block
-        tile_drain(bar, 0);
-        return;
     }
     auto gather = [&](int i, int h) {
         cp_async16(b.st + 2 * (nloc + i), a.q32in + 2 * (size_t)h);
         cp_async16(b.st + 2 * (nloc + i) + 1, a.q32in + 2 * (size_t)h + 1);
     };
-    if (hx0 >= 0) gather(i0, hx0);
-    if (hx1 >= 0) gather(i1, hx1);
-    for (int i = threadIdx.x + 2 * T; i < a.halo_stride; i += T) {
-        const int h = hrow[i];
-        if (h >= 0) gather(i, h);
+    if (!stopped) {
+        if (hx0 >= 0) gather(i0, hx0);
+        if (hx1 >= 0) gather(i1, hx1);
+        for (int i = threadIdx.x + 2 * T; i < a.halo_stride; i += T) {
+            const int h = hrow[i];
+            if (h >= 0) gather(i, h);
+        }
     }
     cp_async_wait_all();
+    __syncthreads();  // the barrier is initialised
     if (!tile_wait(a, bar, 0)) {
         tile_drain(bar, 0);
         return;
     }
+    if (done) return;  // uniform across the block
     const ArgStep sp{a};
     float *fs = reinterpret_cast<float *>(b.rec);
     tile_fluxes_f32<kStageThreads>(a, sp, b, fs, threadIdx.x, nf, c0);
@@ -326,23 +323,28 @@ __device__ __forceinline__ void tile_body_f32(const StageArgs &a, int tile, doub
 }
 
 template <int MINB>
-__global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel_f32(StageArgs a) {
+__global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel_f32(StageArgs a,
+                                                                       const __grid_constant__ CoeffArgs c) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     pdl_release();
-    tile_body_f32(a, blockIdx.x, a.partials + blockIdx.x, smem_raw);
+    const int tile = (int)blockIdx.x - a.force_blocks;
+    if (tile < 0) {
+        pdl_wait();
+        force_block(c, blockIdx.x, a.force_blocks, smem_raw);
+        return;
+    }
+    tile_body_f32(a, tile, a.partials + tile, smem_raw);
 }
 
 // Several solvers in one grid (see tile_batch_kernel).
 template <int MINB>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel_f32(BatchStage bs) {
-    pdl_release();
-    if ((int)blockIdx.x >= *bs.n_entries) {
-        pdl_wait();
-        return;
-    }
-    __shared__ __align__(16) StageArgs sa;
-    const int2 e = batch_stage_args(bs, &sa);
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_release();
+    const int entry = batch_entry(bs, smem_raw);
+    if (entry < 0) return;
+    __shared__ __align__(16) StageArgs sa;
+    const int2 e = batch_stage_args(bs, entry, &sa);
     tile_body_f32(sa, e.y, sa.partials + e.y, smem_raw);
 }
 

@@ -7,8 +7,8 @@ namespace e3d {
 
 // Dynamic shared memory the tile kernels may use (raised before their first launch).
 void prepare_tile_fast(size_t smem_bytes, size_t pipe_smem_bytes) {
-    raise_smem_limit((const void *)tile_kernel<false, 4>, smem_bytes);
-    raise_smem_limit((const void *)tile_kernel<false, 7>, smem_bytes);
+    raise_smem_limit((const void *)tile_kernel<false, 4>, with_forces(smem_bytes, 1));
+    raise_smem_limit((const void *)tile_kernel<false, 7>, with_forces(smem_bytes, 1));
     if (pipe_smem_bytes) raise_smem_limit((const void *)tile_ws_kernel<WS_FAST>, pipe_smem_bytes);
 }
 
@@ -65,17 +65,17 @@ void launch_colour_finish_fast(const StageArgs &a, const double2 *rc, cudaStream
 // variant 0: gather kernel, registers for 4 blocks/SM; 1: gather kernel, 5 blocks/SM;
 // 2: face tiles, one block per tile (4 blocks/SM); 3: face tiles, persistent and warp-specialised;
 // 4: face tiles with registers for 7 blocks/SM
-void launch_stage_fast(const StageArgs &a, cudaStream_t s, int variant) {
+void launch_stage_fast(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant) {
     const int blocks = (a.n_cells + kStageThreads - 1) / kStageThreads;
     if (variant == 4) {
         const size_t smem = tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
-        launch_dependent(tile_kernel<false, 7>, blocks, kStageThreads, smem, s, a);
+        launch_dependent(tile_kernel<false, 7>, blocks + a.force_blocks, kStageThreads, with_forces(smem, a.force_blocks), s, a, c);
     } else if (variant == 3) {
         const size_t smem = ws_smem_for(ws_buffer_bytes(WS_FAST, a.smem_cells, a.smem_faces, a.max_contrib), a.ws_buffers);
         tile_ws_kernel<WS_FAST><<<a.pipe_grid, kWsThreads, smem, s>>>(a);
     } else if (variant == 2) {
         const size_t smem = tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
-        launch_dependent(tile_kernel<false, 4>, blocks, kStageThreads, smem, s, a);
+        launch_dependent(tile_kernel<false, 4>, blocks + a.force_blocks, kStageThreads, with_forces(smem, a.force_blocks), s, a, c);
     } else if (variant == 1) {
         stage_kernel<false, 5><<<blocks, kStageThreads, 0, s>>>(a);
     } else {

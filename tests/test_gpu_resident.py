@@ -215,3 +215,27 @@ def test_exact_rms_is_the_sequential_sum(name, kind):
             total += v
         assert s.rms_history()[0] == np.sqrt(total / n)
     s.close()
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("run", [
+    dict(max_iter=1), dict(max_iter=2), dict(max_iter=7, check_every=4), dict(max_iter=8, check_every=4),
+    dict(max_iter=40, sampling=3), dict(max_iter=33, sampling=11), dict(max_iter=64), dict(max_iter=21, sampling=22),
+    dict(max_iter=400, min_residual_drop=3e-2), dict(max_iter=900, min_aerocoeff_error=2e-4),
+], ids=str)
+@pytest.mark.parametrize("name", ["ogrid", "c1"])
+def test_forces_in_the_first_stage(name, run, precision):
+    """Force coefficients that cannot stop the run are integrated beside the next iteration's first
+    stage (or after the last one): the same samples, wall Cp and stop as with a kernel of their own
+    after every iteration, which the timed runs keep."""
+    arrays = mesh(name)
+    flow = FlowConfig(mach=0.5, aoa=1.0, cfl=1.0, precision=precision, ordering=_lib.ORDER_SPATIAL)
+    state = perturbed_state(arrays, flow, 12, amp=0.02)
+    out = []
+    for profile in (0, 1):
+        s = EulerSolver(arrays, flow, autotune=False)
+        s.set_state(state)
+        stats = s.run(stage_kernel=_lib.KERNEL_TILE, profile_stages=profile, **run)
+        out.append((stats, s.get_state(), s.rms_history(), s.coefficient_history(), s.wall_cp()))
+        s.close()
+    same(*out)
