@@ -32,7 +32,7 @@ namespace e3d {
 // fewest faces is kept.  Parts above kCoarse cells take the estimate's word (a tile's shape is decided
 // by the last few cuts).
 struct TileBisector {
-    static constexpr int kDirs = 16, kCoarse = 1 << 15, kParallel = 1 << 14;
+    static constexpr int kDirs = 16, kCoarse = 1 << 15, kParallel = 1 << 12, kSample = 1 << 10;
     const double *centre;               // 3 per cell
     const int *adj_ptr, *adj, *adj_face;  // interior neighbours of each cell and the faces between
     const double *unit_normal;          // 3 per face
@@ -66,7 +66,7 @@ struct TileBisector {
         double lo[kDirs], hi[kDirs], cost[kDirs] = {};
         std::fill(lo, lo + nd, 1e300);
         std::fill(hi, hi + nd, -1e300);
-        const int stride = coarse ? n / 4096 : n > 8 * tile ? 4 : 1;  // a sample of a large part is enough
+        const int stride = std::max(1, n / kSample);  // a sample of a large part is enough
         for (int i = 0; i < n; i += stride) {
             const int c = cells[i];
             const double *x = centre + 3 * (size_t)c;
@@ -86,9 +86,10 @@ struct TileBisector {
             rank[q] = q;
             cost[q] /= std::max(hi[q] - lo[q], 1e-300);
         }
-        const int tries = std::min(nd, coarse ? 1 : n > 16 * tile ? 2 : 4);
+        int tries = std::min(nd, coarse ? 1 : n > 16 * tile ? 2 : 4);
         std::partial_sort(rank, rank + tries, rank + nd,
                           [&](int a, int b) { return cost[a] < cost[b] || (cost[a] == cost[b] && a < b); });
+        while (tries > 1 && cost[rank[tries - 1]] > 1.6 * cost[rank[0]]) tries--;
         int best = INT_MAX;
         for (int t = 0; t < tries; t++) {
             const double *u = dir[rank[t]];
