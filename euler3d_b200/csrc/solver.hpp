@@ -52,13 +52,14 @@ void launch_batch_ws_f32(const BatchStage &bs, int grid, size_t smem_bytes, cuda
 // Residual smoothing (EulerSolver::smoothResiduals, src/solver/EulerSolver.cpp:483-518): one Jacobi
 // pass over every cell.
 struct SmoothArgs {
-    int n_cells, stride;                 // stride: row stride of the [5 x stride] residual arrays
-    const int *__restrict__ nb_ptr;      // interior neighbours of each cell, element2face order
-    const int *__restrict__ nb;
+    int n_cells, stride;                 // stride: row stride of nb
+    int width;
+    const int *__restrict__ nb;          // [width x stride] interior neighbours of each cell, element2face
+                                         // order, then -1
     const double *__restrict__ den;      // 1 + 0.25 x (faces of the cell, ghosts included)
-    const double *__restrict__ r0;       // the stage's residual
-    const double *__restrict__ last;     // this pass's input
-    double *__restrict__ out;
+    const double2 *r0;                   // the stage's residual (records as StageArgs::r_dev)
+    const double2 *last;                 // this pass's input
+    double2 *__restrict__ out;
     unsigned long long *flags;           // [0] largest change of the first pass (bits), [1] NaN seen
     Control *ctl;
     int pass;                            // 0 first pass, 1 second pass
@@ -70,7 +71,7 @@ void launch_coeff(const CoeffArgs &c, cudaStream_t s);
 void launch_finalize_batch(const FinalizeArgs *f, const int *n_members, int grid, bool exact, cudaStream_t s);
 void launch_coeff_batch(const CoeffArgs *c, const int *n_members, int parity, int grid, cudaStream_t s);
 void launch_control_gather(Control *const *ctl, const int *n_members, Control *out, int grid, cudaStream_t s);
-void launch_smooth(const SmoothArgs &a, cudaStream_t s);
+void launch_smooth(const SmoothArgs &a, bool exact, cudaStream_t s);
 
 template <typename T>
 struct DevBuf {
@@ -136,9 +137,11 @@ struct Solver {
     int sample_cap = 0;
     double wall_sum[3] = {0, 0, 0};
     std::vector<double> wall_center_host;
-    DevBuf<int> nb_ptr, nb;
+    DevBuf<int> nb;
+    int nb_width = 0;
     DevBuf<double> rsq;                 // FP64_EXACT: per-cell R_rho^2 in reference order
-    DevBuf<double> den, rbuf;
+    DevBuf<double> den;
+    DevBuf<double2> rbuf;
     DevBuf<unsigned long long> smooth_flags;
     Control *ctl = nullptr;        // device
     Control *ctl_host = nullptr;   // pinned mirror
@@ -184,8 +187,8 @@ struct Solver {
         q[0].release();
         q[1].release();
         DevBuf<double> *db[] = {&w0, &ecell, &minit, &ghost, &partials, &staging, &wall_svec, &wall_center, &hist,
-                                &scratch, &den, &rbuf};
-        nb_ptr.release();
+                                &scratch, &den};
+        rbuf.release();
         nb.release();
         rsq.release();
         samples.release();
@@ -222,8 +225,8 @@ struct Solver {
                (int64_t)tile_rec32_off.n * 8 +
                (int64_t)(fgeo.n + cgeo.n) * 32 + (int64_t)(q[0].n + q[1].n) * 16 +
                (int64_t)(w0.n + ecell.n + minit.n + ghost.n + partials.n + staging.n + wall_svec.n + wall_center.n +
-                         hist.n + scratch.n + den.n + rbuf.n + smooth_flags.n + samples.n + wall_cp.n + rsq.n) * 8 +
-               (int64_t)(nb_ptr.n + nb.n) * 4 + (int64_t)colour_faces.n * 48 + (int64_t)colour_r.n * 16 +
+                         hist.n + scratch.n + den.n + 2 * rbuf.n + smooth_flags.n + samples.n + wall_cp.n + rsq.n) * 8 +
+               (int64_t)nb.n * 4 + (int64_t)colour_faces.n * 48 + (int64_t)colour_r.n * 16 +
                (int64_t)resident_flags.n * 4 + (int64_t)resident_words.n * 16 +
                (int64_t)sizeof(Control);
     }
@@ -514,23 +517,24 @@ struct Solver {
             launch_stage(a, -1, c);
             return;
         }
-        const size_t n5 = 5 * (size_t)w0_stride;
-        double *r0 = rbuf.p, *r1 = rbuf.p + n5, *r2 = rbuf.p + 2 * n5;
+        const size_t n3 = 3 * (size_t)N;
+        double2 *r0 = rbuf.p, *r1 = rbuf.p + n3, *r2 = rbuf.p + 2 * n3;
+        const bool exact = prm.precision == E3D_PREC_FP64_EXACT;
         StageArgs ar = a;
         ar.split = 1;
         ar.ghost_out = a.last_stage;  // the residual phase of the last stage leaves the ghosts
         ar.last_stage = 0;
         ar.r_dev = r0;
+        ar.smooth_flags = smooth_flags.p;
         launch_stage(ar, -1, c);
-        E3D_CUDA(cudaMemsetAsync(smooth_flags.p, 0, 2 * sizeof(unsigned long long), stream));
-        SmoothArgs sa{N, w0_stride, nb_ptr.p, nb.p, den.p, r0, r0, r1, smooth_flags.p, ctl, 0};
-        launch_smooth(sa, stream);
+        SmoothArgs sa{N, w0_stride, nb_width, nb.p, den.p, r0, r0, r1, smooth_flags.p, ctl, 0};
+        launch_smooth(sa, exact, stream);
         sa.last = r1;
         sa.out = r2;
         sa.pass = 1;
-        launch_smooth(sa, stream);
+        launch_smooth(sa, exact, stream);
         a.r_dev = r2;
-        if (prm.precision == E3D_PREC_FP64_EXACT) launch_update_exact(a, stream);
+        if (exact) launch_update_exact(a, stream);
         else launch_update_fast(a, stream);
     }
 

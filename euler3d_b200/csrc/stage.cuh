@@ -89,8 +89,10 @@ struct alignas(16) StageArgs {  // bulk-copied by tile_ws_batch_kernel
     const float4 *__restrict__ cgeo32;
     int integrator;                  // E3D_INTEGRATOR_RK5 or E3D_INTEGRATOR_EULER (uniform)
     int split;                       // residual phase of a split stage: write R to r_dev, no update
-    double *__restrict__ r_dev;      // [5 x w0_stride] residual of a split stage (device order); the
-                                     // update phase reads the smoothed residual from here
+    double2 *__restrict__ r_dev;     // [3 x n_cells] residual of a split stage (device order, five doubles
+                                     // and a pad per cell, so that a neighbour's is two sectors instead
+                                     // of five); the update phase reads the smoothed residual from here
+    unsigned long long *smooth_flags;  // of the smoothing passes, cleared by the residual phase
     double *__restrict__ rsq;        // FP64_EXACT: R_rho^2 of every cell in reference order (last stage),
                                      // summed sequentially like EulerSolver::computeRMS; else null
     int wait_polls;                  // polls of a tile's data barrier before the wait gives up (kWaitLimit;
@@ -643,9 +645,10 @@ __device__ __forceinline__ double finish_cell(const StageArgs &a, const STEP &sp
         return 0.0;
     }
     if (a.split) {  // residual smoothing runs between this residual and the update
-        const size_t st = (size_t)a.w0_stride;
-#pragma unroll
-        for (int k = 0; k < 5; k++) a.r_dev[k * st + c] = R[k];
+        a.r_dev[3 * (size_t)c] = make_double2(R[0], R[1]);
+        a.r_dev[3 * (size_t)c + 1] = make_double2(R[2], R[3]);
+        a.r_dev[3 * (size_t)c + 2] = make_double2(R[4], 0.0);
+        if (c == 0) a.smooth_flags[0] = a.smooth_flags[1] = 0ull;
         return 0.0;
     }
     double W[5];
@@ -1285,12 +1288,11 @@ __global__ void __launch_bounds__(kStageThreads) update_kernel(StageArgs a) {
     if (c < a.n_cells) {
         const Prim me = load_prim(a.qin, c);
         const size_t st = (size_t)a.w0_stride;
-        double R[5], W0[5];
+        const double2 r0 = a.r_dev[3 * (size_t)c], r1 = a.r_dev[3 * (size_t)c + 1], r2v = a.r_dev[3 * (size_t)c + 2];
+        const double R[5] = {r0.x, r0.y, r1.x, r1.y, r2v.x};
+        double W0[5];
 #pragma unroll
-        for (int k = 0; k < 5; k++) {
-            R[k] = a.r_dev[k * st + c];
-            W0[k] = a.w0[k * st + c];
-        }
+        for (int k = 0; k < 5; k++) W0[k] = a.w0[k * st + c];
         const double r_me = EXACT ? 0.0 : rsqrt_nr(a.gamma * me.p * me.rho);
         Prim out;
         r2 = finish_cell<EXACT>(a, ArgStep{a}, c, me, r_me, R, W0, a.cgeo[c], out);
