@@ -457,6 +457,8 @@ e3d_status e3d_batch_remove(e3d_batch *batch, e3d_solver *solver, e3d_run_stats 
         std::lock_guard<std::mutex> lock(B->mu);
         const int k = B->find(S);
         if (k < 0) throw Error(E3D_ERR_INVALID_ARG, "solver is not a member of this batch");
+        E3D_CUDA(cudaSetDevice(B->device));
+        E3D_CUDA(cudaStreamSynchronize(B->stream));  // its control block, if it was added just now
         B->release(B->members[k], stats);
         B->members.erase(B->members.begin() + k);
         B->dirty = true;

@@ -1,6 +1,7 @@
 // Solver handle of the euler3d_b200 library: device layout construction, the RK5 run loop with
 // on-device stop control, state exchange in the reference's numbering, and the solver half of
 // the C ABI (include/euler3d_b200.h).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -192,118 +193,81 @@ void launch_control_gather(Control *const *ctl, const int *n_members, Control *o
     control_gather_kernel<<<grid, 64, 0, s>>>(ctl, n_members, out);
 }
 
-// Reference-ordered FlowField arrays (staging, 8 x T) -> device layout.
-__global__ void load_state_kernel(const double *__restrict__ st, int64_t T, int n_cells, int n_ghosts,
-                                  const int *__restrict__ new2old, const int *__restrict__ ghost_ref,
-                                  double2 *__restrict__ q, double *__restrict__ w0, int w0_stride,
-                                  double *__restrict__ ecell, double *__restrict__ minit, double *__restrict__ ghost) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t N = (size_t)w0_stride;
-    if (i < n_cells) {
-        int o = new2old[i];
-        double rho = st[o], u = st[T + o], v = st[2 * T + o], w = st[3 * T + o];
-        double p = st[4 * T + o], E = st[5 * T + o], H = st[6 * T + o], M = st[7 * T + o];
-        store_prim(q, i, Prim{rho, u, v, w, p, H});
-        w0[0 * N + i] = rho;  // W0 as RungeKutta forms it (src/solver/EulerSolver.cpp:431-438)
-        w0[1 * N + i] = u * rho;
-        w0[2 * N + i] = v * rho;
-        w0[3 * N + i] = w * rho;
-        w0[4 * N + i] = E * rho;
-        ecell[i] = E;
-        minit[i] = M;
-    } else if (i < n_cells + n_ghosts) {
-        int g = i - n_cells;
-        int r = ghost_ref[g];
-        for (int k = 0; k < 8; k++) ghost[8 * (size_t)g + k] = st[k * T + r];
+// FlowField's eight arrays in the reference's order (rho u v w p E H M, T entries each), in device
+// memory or in pinned host memory that the kernel reads and writes over PCIe.
+struct StateArrays {
+    double *p[8];
+};
+
+// Arrays (or, UNIFORM, one value per array) -> device layout.  One thread per entry in the reference's
+// order, so the arrays are read in whole sectors wherever they are; dev_of: device cell of an interior
+// cell, n_cells + slot of a ghost.
+template <bool F32, bool UNIFORM>
+__global__ void load_state_kernel(StateArrays st, Freestream fs, int64_t T, int n_cells, const int *__restrict__ dev_of,
+                                  double2 *__restrict__ q, float4 *__restrict__ q32, double *__restrict__ w0,
+                                  int w0_stride, double *__restrict__ ecell, double *__restrict__ minit,
+                                  double *__restrict__ ghost, double gamma, Control *ctl) {
+    const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0) {  // a control block of zeros, but the loaded interior Mach holds
+        for (int k = threadIdx.x; k < (int)(sizeof(Control) / 4); k += blockDim.x)
+            reinterpret_cast<int *>(ctl)[k] = k == (int)(offsetof(Control, minit_valid) / 4);
     }
+    if (o >= T) return;
+    double v[8] = {fs.rho, fs.u, fs.v, fs.w, fs.p, fs.E, fs.H, fs.M};
+    if (!UNIFORM)
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = __ldcs(st.p[k] + o);
+    const int i = dev_of[o];
+    if (i >= n_cells) {
+        ghost_store(ghost + 8 * (size_t)(i - n_cells), v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+        return;
+    }
+    const size_t N = (size_t)w0_stride;
+    if (F32) make_rec32(q32 + 2 * (size_t)i, v[0], v[1], v[2], v[3], v[4], v[6], gamma);
+    else store_prim(q, i, Prim{v[0], v[1], v[2], v[3], v[4], v[6]});
+    w0[i] = v[0];  // W0 as RungeKutta forms it (src/solver/EulerSolver.cpp:431-438)
+    w0[N + i] = v[1] * v[0];
+    w0[2 * N + i] = v[2] * v[0];
+    w0[3 * N + i] = v[3] * v[0];
+    w0[4 * N + i] = v[5] * v[0];
+    ecell[i] = v[5];
+    minit[i] = v[7];
 }
 
-// Device layout -> reference-ordered FlowField arrays (staging, 8 x T).  Interior Mach is
-// FlowField's c/|u| (src/solver/FlowField.cpp:157) unless the loaded Mach still holds.
-__global__ void store_state_kernel(double *__restrict__ st, int64_t T, int n_cells, int n_ghosts,
-                                   const int *__restrict__ new2old, const int *__restrict__ ghost_ref,
-                                   const double2 *__restrict__ q, const double *__restrict__ ecell,
-                                   const double *__restrict__ minit, const double *__restrict__ ghost, double gamma,
-                                   const Control *ctl) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n_cells) {
-        int o = new2old[i];
-        Prim s = load_prim(q, i);
-        double M = ctl->minit_valid ? minit[i] : __ddiv_rn(__dsqrt_rn(__dmul_rn(gamma, __ddiv_rn(s.p, s.rho))),
-                                                           __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(s.u, s.u),
-                                                                                          __dmul_rn(s.v, s.v)),
-                                                                                __dmul_rn(s.w, s.w))));
-        st[o] = s.rho;
-        st[T + o] = s.u;
-        st[2 * T + o] = s.v;
-        st[3 * T + o] = s.w;
-        st[4 * T + o] = s.p;
-        st[5 * T + o] = ecell[i];
-        st[6 * T + o] = s.H;
-        st[7 * T + o] = M;
-    } else if (i < n_cells + n_ghosts) {
-        int g = i - n_cells;
-        int r = ghost_ref[g];
-        for (int k = 0; k < 8; k++) st[k * T + r] = ghost[8 * (size_t)g + k];
+// Device layout -> arrays.  Interior Mach is FlowField's c/|u| (src/solver/FlowField.cpp:157) unless the
+// loaded Mach still holds.  FP32_FLUX: the state is the double conservative W0 (updated at every
+// completed RK step).
+template <bool F32>
+__global__ void store_state_kernel(StateArrays st, int64_t T, int n_cells, const int *__restrict__ dev_of,
+                                   const double2 *__restrict__ q, const double *__restrict__ w0, int w0_stride,
+                                   const double *__restrict__ ecell, const double *__restrict__ minit,
+                                   const double *__restrict__ ghost, double gamma, const Control *ctl) {
+    const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (o >= T) return;
+    const int i = dev_of[o];
+    double v[8];
+    if (i >= n_cells) {
+        const double2 *g = reinterpret_cast<const double2 *>(ghost + 8 * (size_t)(i - n_cells));
+        const double2 a = g[0], b = g[1], c = g[2], d = g[3];
+        v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y, v[4] = c.x, v[5] = c.y, v[6] = d.x, v[7] = d.y;
+    } else if (F32) {
+        const size_t N = (size_t)w0_stride;
+        const double rho = w0[i];
+        const double u = w0[N + i] / rho, vv = w0[2 * N + i] / rho, w = w0[3 * N + i] / rho, E = w0[4 * N + i] / rho;
+        const double q2 = u * u + vv * vv + w * w;
+        const double p = (gamma - 1) * rho * (E - q2 / 2.0);
+        v[0] = rho, v[1] = u, v[2] = vv, v[3] = w, v[4] = p, v[5] = E, v[6] = E + p / rho;
+        v[7] = ctl->minit_valid ? minit[i] : sqrt(gamma * (p / rho)) / sqrt(q2);
+    } else {
+        const Prim s = load_prim(q, i);
+        v[0] = s.rho, v[1] = s.u, v[2] = s.v, v[3] = s.w, v[4] = s.p, v[5] = ecell[i], v[6] = s.H;
+        v[7] = ctl->minit_valid ? minit[i]
+                                : __ddiv_rn(__dsqrt_rn(__dmul_rn(gamma, __ddiv_rn(s.p, s.rho))),
+                                            __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(s.u, s.u), __dmul_rn(s.v, s.v)),
+                                                                 __dmul_rn(s.w, s.w))));
     }
-}
-
-// FP32_FLUX mode: reference-ordered FlowField arrays -> float cell records and double W0.
-__global__ void load_state_f32_kernel(const double *__restrict__ st, int64_t T, int n_cells, int n_ghosts,
-                                      const int *__restrict__ new2old, const int *__restrict__ ghost_ref,
-                                      float4 *__restrict__ q32, double *__restrict__ w0, int w0_stride,
-                                      double *__restrict__ ecell, double *__restrict__ minit,
-                                      double *__restrict__ ghost, double gamma) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t N = (size_t)w0_stride;
-    if (i < n_cells) {
-        int o = new2old[i];
-        double rho = st[o], u = st[T + o], v = st[2 * T + o], w = st[3 * T + o];
-        double p = st[4 * T + o], E = st[5 * T + o], H = st[6 * T + o], M = st[7 * T + o];
-        make_rec32(q32 + 2 * (size_t)i, rho, u, v, w, p, H, gamma);
-        w0[0 * N + i] = rho;
-        w0[1 * N + i] = u * rho;
-        w0[2 * N + i] = v * rho;
-        w0[3 * N + i] = w * rho;
-        w0[4 * N + i] = E * rho;
-        ecell[i] = E;
-        minit[i] = M;
-    } else if (i < n_cells + n_ghosts) {
-        int g = i - n_cells;
-        int r = ghost_ref[g];
-        for (int k = 0; k < 8; k++) ghost[8 * (size_t)g + k] = st[k * T + r];
-    }
-}
-
-// FP32_FLUX mode: the state is the double conservative W0 (updated at every completed RK step).
-__global__ void store_state_f32_kernel(double *__restrict__ st, int64_t T, int n_cells, int n_ghosts,
-                                       const int *__restrict__ new2old, const int *__restrict__ ghost_ref,
-                                       const double *__restrict__ w0, int w0_stride,
-                                       const double *__restrict__ minit, const double *__restrict__ ghost,
-                                       double gamma, const Control *ctl) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t N = (size_t)w0_stride;
-    if (i < n_cells) {
-        int o = new2old[i];
-        double rho = w0[i], u = w0[N + i] / rho, v = w0[2 * N + i] / rho, w = w0[3 * N + i] / rho;
-        double E = w0[4 * N + i] / rho;
-        double q2 = u * u + v * v + w * w;
-        double p = (gamma - 1) * rho * (E - q2 / 2.0);
-        double H = E + p / rho;
-        double M = ctl->minit_valid ? minit[i] : sqrt(gamma * (p / rho)) / sqrt(q2);
-        st[o] = rho;
-        st[T + o] = u;
-        st[2 * T + o] = v;
-        st[3 * T + o] = w;
-        st[4 * T + o] = p;
-        st[5 * T + o] = E;
-        st[6 * T + o] = H;
-        st[7 * T + o] = M;
-    } else if (i < n_cells + n_ghosts) {
-        int g = i - n_cells;
-        int r = ghost_ref[g];
-        for (int k = 0; k < 8; k++) st[k * T + r] = ghost[8 * (size_t)g + k];
-    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) __stcs(st.p[k] + o, v[k]);
 }
 
 // ------------------------------------------------------------------------------ host handle
@@ -836,7 +800,10 @@ static void create_solver(const e3d_mesh_desc *d, const e3d_flow_params *p, Solv
     S->fgeo.upload(fgeo, s);
     S->cgeo.upload(cgeo, s);
     S->new2old_d.upload(new2old, s);
-    S->ghost_ref_d.upload(ghost_ref, s);
+    std::vector<int> dev_of((size_t)N + G);
+    for (int c = 0; c < N; c++) dev_of[new2old[c]] = c;
+    for (int g = 0; g < G; g++) dev_of[ghost_ref[g]] = N + g;
+    S->dev_of.upload(dev_of, s);
     S->wall_cell.upload(wcell, s);
     S->wall_svec.upload(wsv, s);
     S->wall_center.upload(wct, s);
@@ -906,39 +873,115 @@ static void create_solver(const e3d_mesh_desc *d, const e3d_flow_params *p, Solv
     E3D_CUDA(cudaStreamSynchronize(s));
 }
 
-static void upload_state(Solver *S, const double *const *arr) {
-    const int64_t T = S->state_size();
-    for (int k = 0; k < 8; k++) {
-        if (!arr[k]) throw Error(E3D_ERR_INVALID_ARG, "state array is NULL");
-        E3D_CUDA(cudaMemcpyAsync(S->staging.p + k * T, arr[k], T * sizeof(double), cudaMemcpyHostToDevice, S->stream));
+// States up to this size go between pinned host memory and the device layout by the kernels' own loads
+// and stores, larger ones through staging by the copy engines: eight copies cost several us each however
+// short, but their rate over PCIe is higher.  set / get, staged against direct: 0.5 MB 80 / 76 against
+// 48 / 45 us, 2.6 MB 120 / 113 against 93 / 86, 4.9 MB 174 / 157 against 141 / 132, 10 MB 262 / 238
+// against 279 / 256, 25 MB equal, 99 MB 1960 / 1920 against 2250 / 2390.
+constexpr size_t kDirectStateBytes = (size_t)6 << 20;
+
+// Device address of `bytes` bytes of pinned host memory at p, or null: not pinned, not mapped, not
+// aligned, or not pinned over the whole range.
+static double *pinned_address(const double *p, size_t bytes) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
     }
-    int threads = 256, blocks = (int)((T + threads - 1) / threads);
-    if (S->f32)
-        load_state_f32_kernel<<<blocks, threads, 0, S->stream>>>(S->staging.p, T, S->N, S->G, S->new2old_d.p,
-                                                                 S->ghost_ref_d.p, S->q32[0].p, S->w0.p,
-                                                                 S->w0_stride, S->ecell.p, S->minit.p, S->ghost.p,
-                                                                 S->prm.gamma);
-    else
-        load_state_kernel<<<blocks, threads, 0, S->stream>>>(S->staging.p, T, S->N, S->G, S->new2old_d.p,
-                                                             S->ghost_ref_d.p, S->q[0].p, S->w0.p, S->w0_stride,
-                                                             S->ecell.p, S->minit.p, S->ghost.p);
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer || reinterpret_cast<uintptr_t>(at.devicePointer) % 8) return nullptr;
+    using Query = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static Query query = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) != cudaSuccess) cudaGetLastError();
+        return found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(fn) : nullptr;
+    }();
+    CUdeviceptr start = 0, at_dev = reinterpret_cast<CUdeviceptr>(at.devicePointer);
+    size_t size = 0;
+    if (!query || query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at_dev) != CUDA_SUCCESS ||
+        query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at_dev) != CUDA_SUCCESS)
+        return nullptr;
+    return at_dev >= start && at_dev + bytes <= start + size ? static_cast<double *>(at.devicePointer) : nullptr;
+}
+
+// The arrays as the kernels can reach them directly; false: through staging.  Outputs that overlap one
+// another go through staging too, whose copies run in order.
+static bool direct_state(const Solver *S, const double *const *arr, bool output, StateArrays &out) {
+    const size_t bytes = (size_t)S->state_size() * sizeof(double);
+    if (8 * bytes > kDirectStateBytes) return false;
+    for (int k = 0; k < 8; k++) {
+        out.p[k] = pinned_address(arr[k], bytes);
+        if (!out.p[k]) return false;
+        for (int j = 0; output && j < k; j++)
+            if ((size_t)std::abs(reinterpret_cast<const char *>(arr[j]) - reinterpret_cast<const char *>(arr[k])) < bytes)
+                return false;
+    }
+    return true;
+}
+
+static StateArrays staged_state(Solver *S) {
+    StateArrays st;
+    for (int k = 0; k < 8; k++) st.p[k] = S->staging.p + k * S->state_size();
+    return st;
+}
+
+template <bool F32, bool UNIFORM>
+static void launch_load_state(Solver *S, const StateArrays &st) {
+    const int64_t T = S->state_size();
+    const int threads = 256, blocks = (int)((T + threads - 1) / threads);
+    load_state_kernel<F32, UNIFORM><<<blocks, threads, 0, S->stream>>>(st, S->fs, T, S->N, S->dev_of.p, S->q[0].p,
+                                                                       S->q32[0].p, S->w0.p, S->w0_stride, S->ecell.p,
+                                                                       S->minit.p, S->ghost.p, S->prm.gamma, S->ctl);
     E3D_CUDA(cudaGetLastError());
+}
+
+// After a state was loaded: buffer 0, and the host's mirror of the control block the kernel wrote.
+static void state_loaded(Solver *S) {
     S->cur = 0;
+    E3D_CUDA(cudaStreamSynchronize(S->stream));
     Control init{};
     init.minit_valid = 1;
     std::memcpy(S->ctl_host, &init, sizeof init);
-    E3D_CUDA(cudaMemcpyAsync(S->ctl, S->ctl_host, sizeof(Control), cudaMemcpyHostToDevice, S->stream));
+}
+
+static void upload_state(Solver *S, const double *const *arr) {
+    const int64_t T = S->state_size();
+    for (int k = 0; k < 8; k++)
+        if (!arr[k]) throw Error(E3D_ERR_INVALID_ARG, "state array is NULL");
+    StateArrays st;
+    if (!direct_state(S, arr, false, st)) {
+        st = staged_state(S);
+        for (int k = 0; k < 8; k++)
+            E3D_CUDA(cudaMemcpyAsync(st.p[k], arr[k], T * sizeof(double), cudaMemcpyHostToDevice, S->stream));
+    }
+    if (S->f32) launch_load_state<true, false>(S, st);
+    else launch_load_state<false, false>(S, st);
+    state_loaded(S);
+}
+
+static void download_state(Solver *S, double *const *arr) {
+    const int64_t T = S->state_size();
+    StateArrays st;
+    const bool direct = direct_state(S, arr, true, st);
+    if (!direct) st = staged_state(S);
+    const int threads = 256, blocks = (int)((T + threads - 1) / threads);
+    if (S->f32)
+        store_state_kernel<true><<<blocks, threads, 0, S->stream>>>(st, T, S->N, S->dev_of.p, nullptr, S->w0.p, S->w0_stride,
+                                                                    S->ecell.p, S->minit.p, S->ghost.p, S->prm.gamma, S->ctl);
+    else
+        store_state_kernel<false><<<blocks, threads, 0, S->stream>>>(st, T, S->N, S->dev_of.p, S->q[S->cur].p, S->w0.p,
+                                                                     S->w0_stride, S->ecell.p, S->minit.p, S->ghost.p,
+                                                                     S->prm.gamma, S->ctl);
+    E3D_CUDA(cudaGetLastError());
+    for (int k = 0; !direct && k < 8; k++)
+        E3D_CUDA(cudaMemcpyAsync(arr[k], st.p[k], T * sizeof(double), cudaMemcpyDeviceToHost, S->stream));
     E3D_CUDA(cudaStreamSynchronize(S->stream));
 }
 
 static void set_freestream(Solver *S) {
-    const int64_t T = S->state_size();
-    std::vector<double> buf(8 * (size_t)T);
-    const double v[8] = {S->fs.rho, S->fs.u, S->fs.v, S->fs.w, S->fs.p, S->fs.E, S->fs.H, S->fs.M};
-    for (int k = 0; k < 8; k++) std::fill(buf.begin() + k * T, buf.begin() + (k + 1) * T, v[k]);
-    const double *arr[8];
-    for (int k = 0; k < 8; k++) arr[k] = buf.data() + k * T;
-    upload_state(S, arr);
+    if (S->f32) launch_load_state<true, true>(S, StateArrays{});
+    else launch_load_state<false, true>(S, StateArrays{});
+    state_loaded(S);
 }
 
 }  // namespace e3d
@@ -956,11 +999,10 @@ static Solver *solo(e3d_solver *s) {
 
 // A fresh control block for a run -- a new EulerSolver's counters (_nbInteration = 0,
 // _CL = _CD = _CM = 0, src/solver/EulerSolver.cpp:21-58) -- keeping whether the loaded interior
-// Mach still holds.  Reads the old block back first (synchronises stream s once).
+// Mach still holds.  The host's mirror has the block as the last call left it: every call that changes
+// it on the device reads it back or knows what it wrote.
 static void init_control(Solver *S, const e3d_run_params *rp, int max_iter, int hist_cap, int sample_cap, bool defer,
                          cudaStream_t s) {
-    E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s));
-    E3D_CUDA(cudaStreamSynchronize(s));
     Control init{};
     init.minit_valid = S->ctl_host->minit_valid;
     init.max_iter = max_iter;
@@ -1124,21 +1166,7 @@ e3d_status e3d_solver_get_state(e3d_solver *solver, double *const state[8]) {
         for (int k = 0; k < 8; k++)
             if (!state[k]) throw Error(E3D_ERR_INVALID_ARG, "state array is NULL");
         E3D_CUDA(cudaSetDevice(S->device));
-        const int64_t T = S->state_size();
-        int threads = 256, blocks = (int)((T + threads - 1) / threads);
-        if (S->f32)
-            store_state_f32_kernel<<<blocks, threads, 0, S->stream>>>(S->staging.p, T, S->N, S->G, S->new2old_d.p,
-                                                                      S->ghost_ref_d.p, S->w0.p, S->w0_stride,
-                                                                      S->minit.p, S->ghost.p, S->prm.gamma, S->ctl);
-        else
-            store_state_kernel<<<blocks, threads, 0, S->stream>>>(S->staging.p, T, S->N, S->G, S->new2old_d.p,
-                                                                  S->ghost_ref_d.p, S->q[S->cur].p, S->ecell.p,
-                                                                  S->minit.p, S->ghost.p, S->prm.gamma, S->ctl);
-        E3D_CUDA(cudaGetLastError());
-        for (int k = 0; k < 8; k++)
-            E3D_CUDA(cudaMemcpyAsync(state[k], S->staging.p + k * T, T * sizeof(double), cudaMemcpyDeviceToHost,
-                                     S->stream));
-        E3D_CUDA(cudaStreamSynchronize(S->stream));
+        download_state(S, state);
     });
 }
 
@@ -1228,6 +1256,7 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
             for (int left = max_iter; left > 0;) {
                 const int n = std::min(every, left);
                 S->launch_resident(n);
+                E3D_CUDA(cudaEventRecord(S->ev1, S->stream));
                 launches++;
                 left -= n;
                 E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, S->stream));
@@ -1257,6 +1286,7 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
                     if (defer) S->enqueue_forces(n & 1);
                     E3D_CUDA(cudaGetLastError());
                 }
+                E3D_CUDA(cudaEventRecord(S->ev1, S->stream));
                 launches += (int64_t)S->kernels_per_iteration(defer) * n + (defer ? 1 : 0);
                 launched_iters += n;
                 E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, S->stream));
@@ -1308,9 +1338,11 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
                 if (S->ctl_host->done) break;
             }
         }
-        E3D_CUDA(cudaEventRecord(S->ev1, S->stream));
-        E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, S->stream));
-        E3D_CUDA(cudaStreamSynchronize(S->stream));
+        if (max_iter == 0 || rp->profile_stages == 1) {  // else recorded and read back with the last launch
+            E3D_CUDA(cudaEventRecord(S->ev1, S->stream));
+            E3D_CUDA(cudaMemcpyAsync(S->ctl_host, S->ctl, sizeof(Control), cudaMemcpyDeviceToHost, S->stream));
+            E3D_CUDA(cudaStreamSynchronize(S->stream));
+        }
         float ms = 0.f;
         E3D_CUDA(cudaEventElapsedTime(&ms, S->ev0, S->ev1));
         const Control &c = *S->ctl_host;

@@ -106,7 +106,7 @@ struct Solver {
 
     std::vector<int> new2old, ghost_ref;  // host copies of the maps
 
-    DevBuf<int> cptr, new2old_d, ghost_ref_d, wall_cell, tile_halo_ptr, tile_halo, tile_face_ptr;
+    DevBuf<int> cptr, new2old_d, dev_of, wall_cell, tile_halo_ptr, tile_halo, tile_face_ptr;
     DevBuf<FaceRec> tile_rec;
     DevBuf<long long> tile_rec_off;
     bool f32 = false;                  // FP32_FLUX mode
@@ -168,7 +168,7 @@ struct Solver {
         for (auto e : prof_ev)
             if (e) cudaEventDestroy(e);
         for (auto e : graph_ev) cudaEventDestroy(e);
-        DevBuf<int> *ib[] = {&cptr, &new2old_d, &ghost_ref_d, &wall_cell, &tile_halo_ptr, &tile_halo, &tile_face_ptr};
+        DevBuf<int> *ib[] = {&cptr, &new2old_d, &dev_of, &wall_cell, &tile_halo_ptr, &tile_halo, &tile_face_ptr};
         for (auto *b : ib) b->release();
         tile_rec.release();
         tile_rec_off.release();
@@ -219,7 +219,7 @@ struct Solver {
     bool colours_built() const { return colour_faces.p != nullptr; }
 
     int64_t device_bytes() const {
-        return (int64_t)(cptr.n + new2old_d.n + ghost_ref_d.n + wall_cell.n + tile_halo_ptr.n + tile_halo.n +
+        return (int64_t)(cptr.n + new2old_d.n + dev_of.n + wall_cell.n + tile_halo_ptr.n + tile_halo.n +
                          tile_face_ptr.n) * 4 + (int64_t)cf.n * 8 + (int64_t)tile_rec.n * 40 + (int64_t)tile_rec_off.n * 8 +
                (int64_t)tile_contrib.n * 2 + (int64_t)(q32[0].n + q32[1].n + cgeo32.n) * 16 + (int64_t)tile_rec32.n * 24 +
                (int64_t)tile_rec32_off.n * 8 +
