@@ -6,7 +6,7 @@ namespace e3d {
 
 void prepare_tile_f32(size_t smem_bytes, size_t ws_smem_bytes) {
     raise_smem_limit((const void *)tile_kernel_f32<4>, with_forces(smem_bytes, 1));
-    raise_smem_limit((const void *)tile_kernel_f32<8>, with_forces(smem_bytes, 1));
+    raise_smem_limit((const void *)tile_kernel_f32<9>, with_forces(smem_bytes, 1));
     if (ws_smem_bytes) raise_smem_limit((const void *)tile_ws_kernel<WS_F32>, ws_smem_bytes);
 }
 
@@ -26,7 +26,9 @@ void launch_batch_f32(const BatchStage &bs, int grid, size_t smem_bytes, cudaStr
 }
 
 // variant 2: face tiles with registers for four blocks/SM; 3: warp-specialised persistent face
-// tiles; 4: face tiles at eight blocks/SM
+// tiles; 4: face tiles at nine blocks/SM (56 registers, no spills; 1.57M tetrahedra 71.7 us a stage at
+// eight blocks, 69.5 at nine, 561k-cell AUSM channel 25.0 and 23.4; the batch kernel spills at nine and
+// takes 141 us an iteration instead of 131, so it stays at eight)
 void launch_stage_f32(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant) {
     const int blocks = (a.n_cells + kStageThreads - 1) / kStageThreads;
     const size_t smem = tile32_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
@@ -34,7 +36,7 @@ void launch_stage_f32(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, in
         const size_t ws = ws_smem_for(ws_buffer_bytes(WS_F32, a.smem_cells, a.smem_faces, a.max_contrib), a.ws_buffers);
         tile_ws_kernel<WS_F32><<<a.pipe_grid, kWsThreads, ws, s>>>(a);
     } else if (variant == 4) {
-        launch_dependent(tile_kernel_f32<8>, blocks + a.force_blocks, kStageThreads, with_forces(smem, a.force_blocks), s, a, c);
+        launch_dependent(tile_kernel_f32<9>, blocks + a.force_blocks, kStageThreads, with_forces(smem, a.force_blocks), s, a, c);
     } else {
         launch_dependent(tile_kernel_f32<4>, blocks + a.force_blocks, kStageThreads, with_forces(smem, a.force_blocks), s, a, c);
     }

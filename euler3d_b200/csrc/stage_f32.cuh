@@ -5,7 +5,7 @@
 // cells, bulk copies of the tile's contiguous data plus cp.async gathers of its halo onto one
 // mbarrier, each face evaluated once, each cell summing its faces' F*S in ascending reference face
 // id (deterministic).  Cell records are 32 bytes (two float4), face records 24 bytes, so a tile's
-// staging is about half the double-precision one and eight blocks fit on an SM.
+// staging is about half the double-precision one and nine blocks fit on an SM.
 #pragma once
 #include "stage.cuh"
 

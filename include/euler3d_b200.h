@@ -219,7 +219,7 @@ typedef struct e3d_run_params {
 	                                     autotuned stage kernel; 1, 2: per-cell gather with two
 	                                     register budgets (FP64 modes); 3: face tiles; 4: persistent
 	                                     face tiles with a producer warp streaming tiles to consumer
-	                                     warps; 5: face tiles at seven blocks per SM (FP64) or eight
+	                                     warps; 5: face tiles at seven blocks per SM (FP64) or nine
 	                                     (FP32_FLUX); 6, 7: face colouring, one launch per class of
 	                                     faces that share no cell, 128 or 512 faces per block (FP64)
 	                                     (kept for later runs) */
