@@ -400,7 +400,7 @@ def run_ours(args, rank, world, local_rank):
                                      "traffic_steady adds the new states' writes still in L2 when the captured "
                                      "launch ended (written back later)",
                      "peak_kind": peak_kind,
-                     "kernel": (["-", "-", "tile_kernel_f32<4>", "tile_ws_kernel<WS_F32>", "tile_kernel_f32<8>", "-", "-"]
+                     "kernel": (["-", "-", "tile_kernel_f32<4>", "tile_ws_kernel<WS_F32>", "tile_kernel_f32<9>", "-", "-"]
                                 if args.precision == "fp32" else
                                 ["stage_kernel<false,4>", "stage_kernel<false,5>", "tile_kernel<false,4>",
                                  "tile_ws_kernel<WS_FAST>", "tile_kernel<false,7>", "colour_kernel<128> (per class)",
@@ -478,7 +478,7 @@ def fp32_flux_leg(arrays, flow, n_cells: int, n_faces: int, K: int, W: int, peak
         err[k] = float(np.max(np.abs(g32[k][:n_cells] - g64[k][:n_cells]) / scale))
     bpc = algorithmic_bytes_per_cell_stage(n_cells, n_faces, fp32=True)
     return {"value": 5.0 * n_cells * K / (ms / 1e3), "unit": UNIT, "ms_per_step": ms / K, "steps": K, "warmup": W,
-            "stage_kernel": ["-", "-", "tile_kernel_f32<4>", "tile_ws_kernel<WS_F32>", "tile_kernel_f32<8>", "-", "-"][variant],
+            "stage_kernel": ["-", "-", "tile_kernel_f32<4>", "tile_ws_kernel<WS_F32>", "tile_kernel_f32<9>", "-", "-"][variant],
             "avg_launch_ms": stage_ms, "bytes_per_cell_stage": bpc,
             "achieved_GBs": bpc * n_cells / (stage_ms / 1e3) / 1e9,
             "frac": bpc * n_cells / (stage_ms / 1e3) / 1e9 / peak,
