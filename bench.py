@@ -53,7 +53,7 @@ def parse():
     ap.add_argument("--ordering", choices=["spatial", "rcm", "native"], default="spatial")
     ap.add_argument("--kernel", type=int, default=0,
                     help="stage kernel: 0 autotuned, 1/2 gather, 3 face tiles, 4 warp-specialised persistent face tiles, "
-                         "5 face tiles at 7 blocks/SM (FP32_FLUX: 8 blocks/SM)")
+                         "5 face tiles at 7 blocks/SM (FP32_FLUX: 9 blocks/SM)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--mode", choices=["all", "stage", "served", "profile", "kernels"], default="all",
