@@ -1278,24 +1278,30 @@ __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel(BatchSt
 
 // ---- update phase of a split stage
 // One thread per cell: the time step and the update of finish_cell from the residual in r_dev
-// (smoothed between the residual phase and this one).  Blocks of kStageThreads cells, so the RMS
+// (smoothed between the residual phase and this one, by kernels that leave state, W0 and geometry alone:
+// those are loaded before it waits for them).  Blocks of kStageThreads cells, so the RMS
 // partials line up with those of the stage kernels.
 template <bool EXACT>
 __global__ void __launch_bounds__(kStageThreads) update_kernel(StageArgs a) {
-    if (a.ctl->done) return;  // uniform across the grid
     const int c = blockIdx.x * kStageThreads + threadIdx.x;
-    double r2 = 0.0;
+    const size_t st = (size_t)a.w0_stride;
+    double r2 = 0.0, W0[5];
+    Prim me;
+    double4 cg;
     if (c < a.n_cells) {
-        const Prim me = load_prim(a.qin, c);
-        const size_t st = (size_t)a.w0_stride;
-        const double2 r0 = a.r_dev[3 * (size_t)c], r1 = a.r_dev[3 * (size_t)c + 1], r2v = a.r_dev[3 * (size_t)c + 2];
-        const double R[5] = {r0.x, r0.y, r1.x, r1.y, r2v.x};
-        double W0[5];
+        me = load_prim(a.qin, c);
 #pragma unroll
         for (int k = 0; k < 5; k++) W0[k] = a.w0[k * st + c];
+        cg = a.cgeo[c];
+    }
+    pdl_wait();
+    if (a.ctl->done) return;  // uniform across the grid
+    if (c < a.n_cells) {
+        const double2 r0 = a.r_dev[3 * (size_t)c], r1 = a.r_dev[3 * (size_t)c + 1], r2v = a.r_dev[3 * (size_t)c + 2];
+        const double R[5] = {r0.x, r0.y, r1.x, r1.y, r2v.x};
         const double r_me = EXACT ? 0.0 : rsqrt_nr(a.gamma * me.p * me.rho);
         Prim out;
-        r2 = finish_cell<EXACT>(a, ArgStep{a}, c, me, r_me, R, W0, a.cgeo[c], out);
+        r2 = finish_cell<EXACT>(a, ArgStep{a}, c, me, r_me, R, W0, cg, out);
     }
     if (a.last_stage) block_sum_store(r2, a.partials + blockIdx.x);
 }

@@ -19,7 +19,7 @@ void prepare_batch_fast(size_t smem_bytes, size_t ws_smem_bytes) {
 
 // Update phase of a split stage (residual smoothing between residual and update).
 void launch_update_fast(const StageArgs &a, cudaStream_t s) {
-    update_kernel<false><<<(a.n_cells + kStageThreads - 1) / kStageThreads, kStageThreads, 0, s>>>(a);
+    launch_dependent(update_kernel<false>, (a.n_cells + kStageThreads - 1) / kStageThreads, kStageThreads, 0, s, a);
 }
 
 // One stage of every member of a batch: `grid` blocks over the (member, tile) table.
