@@ -1099,6 +1099,13 @@ __device__ __forceinline__ double tile_update(const StageArgs &a, const STEP &sp
 #pragma unroll
         for (int q = 0; q < 5; q++) R[q] = fma(sg, fs[5 * j + q], R[q]);
     }
+    for (int k = 6; k < a.max_contrib; k++) {  // cells of more faces than the element types have
+        const unsigned x = b.ct[k * T + i];
+        if (x == kNoContrib) break;
+        const double sg = (x & 1) ? -1.0 : 1.0;
+#pragma unroll
+        for (int q = 0; q < 5; q++) R[q] = fma(sg, fs[5 * (int)(x >> 1) + q], R[q]);
+    }
     return finish_cell<EXACT>(a, sp, c0 + i, me, EXACT ? 0.0 : rsqrt_nr(a.gamma * me.p * me.rho), R, W0, cg, out);
 }
 

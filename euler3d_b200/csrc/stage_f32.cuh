@@ -212,6 +212,13 @@ __device__ __forceinline__ double tile_update_f32(const StageArgs &a, const STEP
 #pragma unroll
         for (int q = 0; q < 5; q++) R[q] = fma(sg, (double)fs[6 * j + q], R[q]);
     }
+    for (int k = 6; k < MC; k++) {  // cells of more faces than the element types have
+        const unsigned x = b.ct[k * T + i];
+        if (x == kNoContrib) break;
+        const double sg = (x & 1) ? -1.0 : 1.0;
+#pragma unroll
+        for (int q = 0; q < 5; q++) R[q] = fma(sg, (double)fs[6 * (int)(x >> 1) + q], R[q]);
+    }
     // time step in single precision (TimeStepMethod2, src/solver/TimeIntegration.cpp:8-40)
     const float snd = gf * me.p * me.r;
     const float lam = 0.5f * fmaf(fabsf(me.u) + snd, cg.x, fmaf(fabsf(me.v) + snd, cg.y, (fabsf(me.w) + snd) * cg.z));
