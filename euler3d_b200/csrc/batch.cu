@@ -316,6 +316,13 @@ struct Batch {
         return E3D_OK;
     }
 
+    // What e3d_batch_add queued on the batch's stream for a member that no step has run since -- its
+    // control block, the wall Cp, the state moved to buffer 0 -- is done before the solver, which has a
+    // stream of its own, is handed back.
+    void settle(const Member &m) const {
+        if (m.iters == 0) E3D_CUDA(cudaStreamSynchronize(stream));
+    }
+
     int find(const Solver *S) const {
         for (size_t k = 0; k < members.size(); k++)
             if (members[k].S == S) return (int)k;
@@ -331,6 +338,7 @@ void batch_detach(Solver *S) {
     std::lock_guard<std::mutex> lock(B->mu);
     const int k = B->find(S);
     if (k >= 0) {
+        cudaStreamSynchronize(B->stream);
         B->release(B->members[k], nullptr);
         B->members.erase(B->members.begin() + k);
         B->dirty = true;
@@ -433,6 +441,7 @@ e3d_status e3d_batch_retire(e3d_batch *batch, e3d_solver **solvers, e3d_run_stat
         keep.reserve(B->members.size());
         for (Member &m : B->members) {
             if (m.stopped && n < capacity) {
+                B->settle(m);
                 solvers[n] = reinterpret_cast<e3d_solver *>(m.S);
                 const e3d_status st = B->release(m, stats ? stats + n : nullptr);
                 if (status) status[n] = st;
@@ -458,7 +467,7 @@ e3d_status e3d_batch_remove(e3d_batch *batch, e3d_solver *solver, e3d_run_stats 
         const int k = B->find(S);
         if (k < 0) throw Error(E3D_ERR_INVALID_ARG, "solver is not a member of this batch");
         E3D_CUDA(cudaSetDevice(B->device));
-        E3D_CUDA(cudaStreamSynchronize(B->stream));  // its control block, if it was added just now
+        B->settle(B->members[k]);
         B->release(B->members[k], stats);
         B->members.erase(B->members.begin() + k);
         B->dirty = true;
