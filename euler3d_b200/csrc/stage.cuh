@@ -194,6 +194,11 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
     return fma(y * e, fma(0.375, e, 0.5), y);  // y (1 + e/2 + 3e^2/8)
 }
 
+// x, made negative where y is: the argument of a root that has to be NaN for a negative y too.
+__device__ __forceinline__ double sign_or(double x, double y) {
+    return __hiloint2double(__double2hiint(x) | (__double2hiint(y) & (int)0x80000000u), __double2loint(x));
+}
+
 // ------------------------------------------------------------------------------ Roe flux
 // Exact: Solver::Roe (src/solver/ConvectiveFluxesSchemes.cpp:10-165) operation by operation.
 __device__ __forceinline__ void roe_exact(const Prim &L, const Prim &R, double nx, double ny, double nz,
@@ -257,14 +262,14 @@ __device__ __forceinline__ void roe_exact(const Prim &L, const Prim &R, double n
 // c_L / 15 needs a root only where the fix applies: |lambda| > delta is tested as 225 rho_L lambda^2 >
 // gamma p_L for the smaller |lambda| = ||V~| - c~|, and the fix is continuous at equality, so a
 // rounding-level difference there is one of the result too (a negative pressure takes the root, so
-// that it still ends in a NaN).
+// that it still ends in a NaN, as a negative density on either side does).
 // The FP64 kernels are compiled without multiply-add contraction and fuse where the source says
 // fma(), so the rounding is fixed by the source: every kernel variant, alone or batched, computes
 // the same bits whatever its register budget.
 __device__ __forceinline__ void roe_fast(const Prim &L, const Prim &R, double nx, double ny, double nz, double g,
                                          double F[5]) {
     const double rr = L.rho * R.rho;
-    const double rt = rr * rsqrt_nr(rr);
+    const double rt = rr * rsqrt_nr(sign_or(rr, L.rho));  // NaN also where both densities are negative
     const double inv = rcp_nr(L.rho + rt);
     double wl = L.rho * inv, wr = rt * inv;
     double ut = fma(L.u, wl, R.u * wr);
@@ -386,7 +391,7 @@ __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double n
     } else {
         const double qt2 = fma(-V, V, fma(d.u, d.u, fma(d.v, d.v, d.w * d.w)));
         const double c2 = (g - 1.0) * fma(-0.5, qt2, d.H);
-        f = fma(d.rho * V, V + c2 * rsqrt_nr(c2), d.p);
+        f = fma(d.rho * V, V + c2 * rsqrt_nr(sign_or(c2, d.rho)), d.p);  // NaN for a negative density
     }
     F[0] = 0.0;
     F[1] = f * nx;

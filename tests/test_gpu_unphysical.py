@@ -1,0 +1,63 @@
+"""States with negative densities and pressures, which a run that is about to fail passes through: the
+FP64 and FP32_FLUX modes' restructured operations end in a NaN where the reference's do."""
+import numpy as np
+import pytest
+
+from cases import CASES, perturbed_state, prepared
+from euler3d_b200 import _lib
+from euler3d_b200.solver import EulerSolver, FlowConfig
+
+pytestmark = pytest.mark.gpu
+
+DOUBLE_KERNELS = [_lib.KERNEL_GATHER, _lib.KERNEL_TILE, _lib.KERNEL_TILE_PIPE, _lib.KERNEL_TILE_B3, _lib.KERNEL_COLOUR]
+
+
+def negated(state, cells):
+    """Density and pressure of `cells` with the other sign, E and H as they were (p / rho is)."""
+    out = {k: v.copy() for k, v in state.items()}
+    for k in ("rho", "p"):
+        out[k][cells] *= -1.0
+    return out
+
+
+def residual(arrays, flow, state, kernel):
+    s = EulerSolver(arrays, flow, autotune=False)
+    s.run(0, stage_kernel=kernel)
+    s.set_state(state)
+    r, _ = s.residual()
+    s.close()
+    return r
+
+
+@pytest.mark.parametrize("kernel", DOUBLE_KERNELS)
+@pytest.mark.parametrize("name", ["channel", "ogrid", "tets"])
+def test_negative_everywhere(name, kernel):
+    arrays = prepared(name)
+    flow = dict(mach=0.5, cfl=1.0, ordering=_lib.ORDER_SPATIAL)
+    state = perturbed_state(arrays, FlowConfig(**flow), 3)
+    state = negated(state, slice(0, int(arrays["n_cells"])))
+    assert np.isnan(residual(arrays, FlowConfig(precision=_lib.PREC_FP64_EXACT, **flow), state, _lib.KERNEL_TILE)).all()
+    assert np.isnan(residual(arrays, FlowConfig(precision=_lib.PREC_FP64, **flow), state, kernel)).all()
+
+
+def cube():
+    """One unit cube, every face a symmetry face."""
+    unit = np.array([[-1, 0, 0], [1, 0, 0], [0, -1, 0], [0, 1, 0], [0, 0, -1], [0, 0, 1]], float)
+    f = np.arange(6, dtype=np.int32)
+    return {"n_cells": 1, "n_faces": 6, "n_faces_int": 0, "face2cell": np.stack([0 * f, 1 + f], 1).ravel(),
+            "face_unit_normal": unit.ravel(), "face_normal": unit.ravel(), "face_area": np.ones(6),
+            "face_center": (0.5 + 0.5 * unit).ravel(), "cell_volume": np.ones(1),
+            "cell2face_ptr": np.array([0, 6], np.int32), "cell2face": f,
+            "sym_face": f, "sym_interior": 0 * f, "sym_ghost": 1 + f}
+
+
+@pytest.mark.parametrize("kernel", DOUBLE_KERNELS)
+@pytest.mark.parametrize("sign", [1, -1])
+def test_symmetry_faces_alone(sign, kernel):
+    arrays = cube()
+    flow = dict(mach=0.5, cfl=1.0)
+    state = perturbed_state(arrays, FlowConfig(**flow), 3)
+    state = negated(state, slice(0, 1)) if sign < 0 else state
+    exact = residual(arrays, FlowConfig(precision=_lib.PREC_FP64_EXACT, **flow), state, _lib.KERNEL_TILE)
+    fast = residual(arrays, FlowConfig(precision=_lib.PREC_FP64, **flow), state, kernel)
+    assert np.isnan(exact[0, 1:4]).all() == np.isnan(fast[0, 1:4]).all() == (sign < 0)
