@@ -452,7 +452,7 @@ __device__ __forceinline__ void ghost_mirror(double *gp, double g, const Prim &d
     double v = d.v - 2 * V * ny;
     double w = d.w - 2 * V * nz;
     if (store) {
-        const double c = PREC == PREC_EXACT ? sqrt(g * (d.p / d.rho)) : d.rho * rsqrt_nr(g * d.p * d.rho);
+        const double c = PREC == PREC_EXACT ? sqrt(g * (d.p / d.rho)) : fabs(d.rho) * rsqrt_nr(g * d.p * d.rho);
         ghost_finish<PREC>(gp, g, d.rho, u, v, w, d.p, c, out);
     } else {
         double H = 0.0;
@@ -507,8 +507,8 @@ __device__ __forceinline__ void ghost_farfield(double *gp, double g, const Frees
         }
         ghost_finish<PREC>(gp, g, rho, u, v, w, p, c, out);
     } else {
-        // with r = 1 / sqrt(gamma p rho): 1/c = rho r, 1/(rho c) = r, rho c = gamma p rho r
-        const double gpr = g * d.p * d.rho, r = rsqrt_nr(gpr), ic = d.rho * r;
+        // with r = 1 / sqrt(gamma p rho), of the density's sign: 1/c = rho r, 1/(rho c) = r, rho c = gamma p rho r
+        const double gpr = g * d.p * d.rho, r = copysign(rsqrt_nr(gpr), d.rho), ic = d.rho * r;
         double p, rho, u, v, w;
         if (V > 0.0) {
             const double dpr = (d.p - fs.p) * r;

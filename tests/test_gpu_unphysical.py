@@ -61,3 +61,27 @@ def test_symmetry_faces_alone(sign, kernel):
     exact = residual(arrays, FlowConfig(precision=_lib.PREC_FP64_EXACT, **flow), state, _lib.KERNEL_TILE)
     fast = residual(arrays, FlowConfig(precision=_lib.PREC_FP64, **flow), state, kernel)
     assert np.isnan(exact[0, 1:4]).all() == np.isnan(fast[0, 1:4]).all() == (sign < 0)
+
+
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_FP32_FLUX])
+@pytest.mark.parametrize("name", ["channel", "ogrid", "tets"])
+def test_ghosts_of_negative_cells(name, precision):
+    """Ghost records of cells whose density and pressure are both negative (the reference's sound speed
+    is a number there), of every boundary kind: the exact mode's, within 30 roundings that the mixed
+    signs magnify up to 30 times (2^-53, or 2^-24 of FP32_FLUX's cell states)."""
+    arrays = prepared(name)
+    n = int(arrays["n_cells"])
+    base = perturbed_state(arrays, FlowConfig(mach=0.5), 3)
+    cells = np.flatnonzero(np.random.default_rng(5).uniform(size=n) < 0.5)
+    got = []
+    for prec in (_lib.PREC_FP64_EXACT, precision):
+        flow = FlowConfig(mach=0.5, cfl=1.0, precision=prec, ordering=_lib.ORDER_SPATIAL)
+        s = EulerSolver(arrays, flow, autotune=False)
+        s.set_state(negated(base, cells))
+        s.residual()
+        got.append(s.get_state())
+        s.close()
+    tol = 900 * (2.0 ** -53 if precision == _lib.PREC_FP64 else 2.0 ** -24)
+    for k in ("rho", "u", "v", "w", "p", "E", "H", "M"):
+        want, have = got[0][k][n:], got[1][k][n:]
+        assert np.max(np.abs(have - want)) <= tol * np.max(np.abs(want)), k
