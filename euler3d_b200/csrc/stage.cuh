@@ -430,7 +430,7 @@ __device__ __forceinline__ void ghost_finish(double *gp, double g, double rho, d
     } else {
         const double q2 = fma(u, u, fma(v, v, w * w));
         const double e = p * rcp_nr((g - 1.0) * rho);  // internal energy; p / rho = (gamma - 1) e
-        M = q2 == 0.0 ? 0.0 : q2 * rsqrt_nr(q2) * c;
+        M = (q2 == 0.0 ? 0.0 : q2 * rsqrt_nr(q2)) * c;
         E = fma(0.5, q2, e);
         H = fma(g - 1.0, e, E);
     }

@@ -85,3 +85,19 @@ def test_ghosts_of_negative_cells(name, precision):
     for k in ("rho", "u", "v", "w", "p", "E", "H", "M"):
         want, have = got[0][k][n:], got[1][k][n:]
         assert np.max(np.abs(have - want)) <= tol * np.max(np.abs(want)), k
+
+
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_FP32_FLUX])
+def test_ghost_mach_of_a_fluid_at_rest(precision):
+    """No velocity and a negative pressure: the ghost's Mach number is 0 / NaN."""
+    arrays = cube()
+    state = perturbed_state(arrays, FlowConfig(mach=0.5), 3)
+    for k in "uvw":
+        state[k][:] = 0.0
+    state["p"][0] = -1.0
+    for prec in (_lib.PREC_FP64_EXACT, precision):
+        s = EulerSolver(arrays, FlowConfig(mach=0.5, precision=prec), autotune=False)
+        s.set_state(state)
+        s.residual()
+        assert np.isnan(s.get_state()["M"][1:]).all()
+        s.close()
