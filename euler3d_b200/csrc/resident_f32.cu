@@ -6,8 +6,8 @@ namespace e3d {
 
 int resident_max_blocks_f32(int shape, size_t smem) { return ResidentLaunch<PREC_F32>::max_blocks(shape, smem); }
 
-void launch_resident_f32(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s) {
-    ResidentLaunch<PREC_F32>::launch(a, r, shape, smem, s);
+bool launch_resident_f32(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s) {
+    return ResidentLaunch<PREC_F32>::launch(a, r, shape, smem, s);
 }
 
 }  // namespace e3d

@@ -888,6 +888,28 @@ static void create_solver(const e3d_mesh_desc *d, const e3d_flow_params *p, Solv
 // against 279 / 256, 25 MB equal, 99 MB 1960 / 1920 against 2250 / 2390.
 constexpr size_t kDirectStateBytes = (size_t)6 << 20;
 
+// A function of the driver's own interface, or null.
+template <typename F>
+static F driver_function(const char *name) {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &found) != cudaSuccess) cudaGetLastError();
+    return found == cudaDriverEntryPointSuccess ? reinterpret_cast<F>(fn) : nullptr;
+}
+
+// SMs that kernels on a stream may use: the device's, or those of the green context it belongs to.
+int stream_sms(cudaStream_t s, int device_sms) {
+    static const auto green_ctx = driver_function<CUresult (*)(CUstream, CUgreenCtx *)>("cuStreamGetGreenCtx");
+    static const auto resource =
+        driver_function<CUresult (*)(CUgreenCtx, CUdevResource *, CUdevResourceType)>("cuGreenCtxGetDevResource");
+    CUgreenCtx ctx = nullptr;
+    CUdevResource r{};
+    if (!green_ctx || !resource || green_ctx(reinterpret_cast<CUstream>(s), &ctx) != CUDA_SUCCESS || !ctx ||
+        resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+        return device_sms;
+    return std::min(device_sms, (int)r.sm.smCount);
+}
+
 // Device address of `bytes` bytes of pinned host memory at p, or null: not pinned, not mapped, not
 // aligned, or not pinned over the whole range.
 static double *pinned_address(const double *p, size_t bytes) {
@@ -897,13 +919,8 @@ static double *pinned_address(const double *p, size_t bytes) {
         return nullptr;
     }
     if (at.type != cudaMemoryTypeHost || !at.devicePointer || reinterpret_cast<uintptr_t>(at.devicePointer) % 8) return nullptr;
-    using Query = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
-    static Query query = [] {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) != cudaSuccess) cudaGetLastError();
-        return found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(fn) : nullptr;
-    }();
+    static const auto query =
+        driver_function<CUresult (*)(void *, CUpointer_attribute, CUdeviceptr)>("cuPointerGetAttribute");
     CUdeviceptr start = 0, at_dev = reinterpret_cast<CUdeviceptr>(at.devicePointer);
     size_t size = 0;
     if (!query || query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at_dev) != CUDA_SUCCESS ||
@@ -1254,16 +1271,16 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
         // kernel's control block has its own way, and timed stages hold nothing else).
         const bool defer = !resident.owns_lock() && rp->profile_stages == 0 && S->can_defer() && !forces_decide(rp);
         begin_run(S, rp, defer, S->stream);
-        if (resident.owns_lock()) {
-            // every tile resident: whole iterations in one launch.  The host looks at the stop flag as
-            // often as the caller asks, otherwise every kResidentIterations (a launch costs less than
-            // one of them, and each ends on state buffer 0)
+        // Every tile resident: whole iterations in one launch.  The host looks at the stop flag as often as
+        // the caller asks, otherwise every kResidentIterations (a launch costs less than one of them, and
+        // each ends on state buffer 0).  False, with nothing launched: the stage kernels do it.
+        auto run_resident = [&] {
             int every = rp->check_every > 0 ? rp->check_every : kResidentIterations;
             every += every & 1;
             E3D_CUDA(cudaEventRecord(S->ev0, S->stream));
             for (int left = max_iter; left > 0;) {
                 const int n = std::min(every, left);
-                S->launch_resident(n);
+                if (!S->launch_resident(n)) return false;
                 E3D_CUDA(cudaEventRecord(S->ev1, S->stream));
                 launches++;
                 left -= n;
@@ -1272,6 +1289,10 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
                 if (S->ctl_host->done || S->ctl_host->fault) break;
                 if (left == 0) throw Error(E3D_ERR_TIMEOUT, "run did not reach its stop condition");
             }
+            return true;
+        };
+        if (resident.owns_lock() && run_resident()) {
+            resident.unlock();
         } else if (rp->profile_stages != 1) {
             int every = rp->check_every > 0 ? rp->check_every : 32;
             every += every & 1;  // whole graphs start and end on buffer 0

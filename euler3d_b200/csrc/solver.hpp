@@ -29,12 +29,13 @@ void launch_colour_fast(const StageArgs &a, const ColourFace *faces, int n, doub
 void launch_colour_finish_fast(const StageArgs &a, const double2 *rc, cudaStream_t s);
 struct Solver;
 void build_colours(Solver *S);
+int stream_sms(cudaStream_t s, int device_sms);
 int resident_max_blocks_exact(int shape, size_t smem);
 int resident_max_blocks_fast(int shape, size_t smem);
 int resident_max_blocks_f32(int shape, size_t smem);
-void launch_resident_exact(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
-void launch_resident_fast(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
-void launch_resident_f32(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
+bool launch_resident_exact(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
+bool launch_resident_fast(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
+bool launch_resident_f32(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s);
 
 void launch_update_exact(const StageArgs &a, cudaStream_t s);
 void launch_fast_reciprocals(const double *x, int64_t n, double *out, cudaStream_t s);
@@ -294,21 +295,23 @@ struct Solver {
     DevBuf<uint4> resident_words;
     unsigned resident_tag = 1;
 
-    // The largest block size at which every tile and the control block are resident together.
+    // The largest block size at which every tile and the control block are resident together, on the SMs
+    // that the solver's stream may use.
     void plan_resident() {
         resident_planned = true;
         if (!tiles_ok || smoothing) return;
         const int prec = f32 ? PREC_F32 : prm.precision == E3D_PREC_FP64 ? PREC_FAST : PREC_EXACT;
         size_t smem = resident_smem_bytes(prec, smem_cells, smem_faces, max_contrib, max_far, n_tiles);
+        const int sms = stream_sms(stream, n_sm);
         // exact mode with a block per SM: room for R_rho^2 of every cell in the control block
         const size_t with_rsq = std::max(smem, kControlHead + 8 * (size_t)N);
-        if (prec == PREC_EXACT && n_tiles < n_sm && with_rsq <= 226 * 1024) smem = with_rsq;
+        if (prec == PREC_EXACT && n_tiles < sms && with_rsq <= 226 * 1024) smem = with_rsq;
         if (smem > 226 * 1024) return;
         for (int shape = 0; shape < kResidentShapeCount; shape++) {
             const int per_sm = prec == PREC_F32    ? resident_max_blocks_f32(shape, smem)
                                : prec == PREC_FAST ? resident_max_blocks_fast(shape, smem)
                                                    : resident_max_blocks_exact(shape, smem);
-            if ((int64_t)per_sm * n_sm < n_tiles + 1) continue;
+            if ((int64_t)per_sm * sms < n_tiles + 1) continue;
             resident_shape = shape;
             resident_smem = smem;
             return;
@@ -334,8 +337,9 @@ struct Solver {
         return true;
     }
 
-    // `iters` iterations from state buffer 0 with the resident kernel.
-    void launch_resident(int iters) {
+    // `iters` iterations from state buffer 0 with the resident kernel; false (and never again): they do
+    // not fit after all.
+    bool launch_resident(int iters) {
         E3D_CUDA(cudaMemsetAsync(resident_flags.p, 0, resident_flags.n * sizeof(unsigned), stream));
         const StageArgs a = stage_args(0, 0.0, 0, 0);
         ResidentArgs r{};
@@ -354,9 +358,11 @@ struct Solver {
         r.max_far = max_far;
         r.stage_rsq = resident_smem >= kControlHead + 8 * (size_t)N;
         r.fin = finalize_args(partials.p, hist.p);
-        if (f32) launch_resident_f32(a, r, resident_shape, resident_smem, stream);
-        else if (prm.precision == E3D_PREC_FP64) launch_resident_fast(a, r, resident_shape, resident_smem, stream);
-        else launch_resident_exact(a, r, resident_shape, resident_smem, stream);
+        const bool ok = f32                                  ? launch_resident_f32(a, r, resident_shape, resident_smem, stream)
+                        : prm.precision == E3D_PREC_FP64 ? launch_resident_fast(a, r, resident_shape, resident_smem, stream)
+                                                         : launch_resident_exact(a, r, resident_shape, resident_smem, stream);
+        if (!ok) resident_shape = -1;
+        return ok;
     }
 
     int variant = 0;                // stage-kernel variant picked by autotune()

@@ -468,10 +468,17 @@ struct ResidentLaunch {
         E3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel(shape), kResidentShapes[shape].threads, smem));
         return n;
     }
-    static void launch(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s) {
+    // False: the GPU, or the part of it that the stream may use, does not hold the grid at once.
+    static bool launch(const StageArgs &a, const ResidentArgs &r, int shape, size_t smem, cudaStream_t s) {
         void *args[] = {const_cast<StageArgs *>(&a), const_cast<ResidentArgs *>(&r)};
-        E3D_CUDA(cudaLaunchCooperativeKernel(kernel(shape), dim3(a.n_tiles + 1), dim3(kResidentShapes[shape].threads), args,
-                                             smem, s));
+        const cudaError_t e = cudaLaunchCooperativeKernel(kernel(shape), dim3(a.n_tiles + 1),
+                                                          dim3(kResidentShapes[shape].threads), args, smem, s);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            cudaGetLastError();
+            return false;
+        }
+        E3D_CUDA(e);
+        return true;
     }
 };
 
