@@ -47,7 +47,6 @@
 namespace e3d {
 
 constexpr int kFlagStride = 8;          // words between two tiles' flags: a 32-byte sector each
-constexpr int kFlagPolls = 1 << 22;     // polls of a flag (about 0.5 us each) before the wait gives up
 constexpr int kResidentIterations = 256;  // per launch, unless the caller asks for more frequent checks
 constexpr unsigned kStopBit = 1u << 31;
 
@@ -115,10 +114,11 @@ __device__ __forceinline__ void store_release(unsigned *p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Bounded wait until the word (without its stop bit) reaches v; false when it gives up or the run was
-// aborted.  got: the word seen.
-__device__ __forceinline__ bool wait_word(const unsigned *word, unsigned v, const unsigned *abort, unsigned &got) {
-    for (int n = 0; n < kFlagPolls; n++) {
+// Bounded wait (`polls` looks of about 0.5 us, StageArgs::wait_polls) until the word (without its stop
+// bit) reaches v; false when it gives up or the run was aborted.  got: the word seen.
+__device__ __forceinline__ bool wait_word(const unsigned *word, unsigned v, const unsigned *abort, int polls,
+                                          unsigned &got) {
+    for (int n = 0; n < polls; n++) {
         got = load_acquire(word);
         if ((got & ~kStopBit) >= v) return true;
         if ((n & 31) == 31 && load_acquire(abort)) return false;
@@ -128,8 +128,8 @@ __device__ __forceinline__ bool wait_word(const unsigned *word, unsigned v, cons
 
 // Bounded wait until all K words at p carry the tag.
 template <int K>
-__device__ __forceinline__ bool wait_words(const uint4 *p, unsigned tag, const unsigned *abort, uint4 w[K]) {
-    for (int n = 0; n < kFlagPolls; n++) {
+__device__ __forceinline__ bool wait_words(const uint4 *p, unsigned tag, const unsigned *abort, int polls, uint4 w[K]) {
+    for (int n = 0; n < polls; n++) {
         bool all = true;
 #pragma unroll
         for (int k = 0; k < K; k++) w[k] = load_word(p + k);
@@ -188,7 +188,7 @@ __device__ __noinline__ void resident_control(const StageArgs &a, const Resident
             unsigned got;
             bool ok = true;
             for (int t = tid; t < a.n_tiles && ok; t += NT)
-                ok = wait_word(r.flags + (size_t)t * kFlagStride, (unsigned)it, abort, got);
+                ok = wait_word(r.flags + (size_t)t * kFlagStride, (unsigned)it, abort, a.wait_polls, got);
             return ok;
         };
         bool ok = true;
@@ -197,7 +197,7 @@ __device__ __noinline__ void resident_control(const StageArgs &a, const Resident
         } else {
             for (int t = tid; t < a.n_tiles && ok; t += NT) {
                 uint4 w[1];
-                ok = wait_words<1>(r.partials + t, r.tag + (unsigned)(it * r.stages), abort, w);
+                ok = wait_words<1>(r.partials + t, r.tag + (unsigned)(it * r.stages), abort, a.wait_polls, w);
                 room[t] = __hiloint2double((int)w[0].y, (int)w[0].x);
             }
         }
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(NT, MINB) resident_kernel(const __grid_constan
             return true;
         }
         uint4 w[kWords];
-        if (!wait_words<kWords>(r.words + (v & 1) * slot + (size_t)h * kWords, r.tag + v, abort, w)) return false;
+        if (!wait_words<kWords>(r.words + (v & 1) * slot + (size_t)h * kWords, r.tag + v, abort, a.wait_polls, w)) return false;
         uint4 *dst = reinterpret_cast<uint4 *>(st_p + (size_t)(nloc + i) * kState);
         dst[0] = make_uint4(w[0].x, w[0].y, w[0].z, w[1].x);
         dst[1] = make_uint4(w[1].y, w[1].z, w[2].x, w[2].y);
@@ -324,8 +324,8 @@ __global__ void __launch_bounds__(NT, MINB) resident_kernel(const __grid_constan
         }
         if (it && tid == 0) {
             unsigned decided = 0, forces;
-            ok = wait_word(words + WORD_DECIDED * kFlagStride, it, abort, decided) && ok;
-            if (ok && !(decided & kStopBit)) ok = wait_word(words + WORD_FORCES * kFlagStride, it, abort, forces);
+            ok = wait_word(words + WORD_DECIDED * kFlagStride, it, abort, a.wait_polls, decided) && ok;
+            if (ok && !(decided & kStopBit)) ok = wait_word(words + WORD_FORCES * kFlagStride, it, abort, a.wait_polls, forces);
             s_word = decided;
         }
         return !__syncthreads_or(!ok);

@@ -295,8 +295,8 @@ class EulerSolver:
         return stats, hist[: st.n_rms].copy()
 
     def set_wait_limit(self, polls: int) -> None:
-        """``e3d_solver_set_wait_limit``: polls of the stage kernels' bounded data waits (negative:
-        the default).  0 makes every wait give up at once, which exercises the timeout path."""
+        """``e3d_solver_set_wait_limit``: polls of the kernels' bounded waits (negative: the
+        default).  0 makes every wait give up at once, which exercises the timeout path."""
         check(_lib.load().e3d_solver_set_wait_limit(self._h, polls))
 
     def rms_history(self) -> np.ndarray:

@@ -271,13 +271,14 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *params, e3d_
 e3d_status e3d_solver_run_noalloc(e3d_solver *solver, const e3d_run_params *params, e3d_run_stats *stats,
                                   double *rms_history, int32_t history_capacity);
 
-/* Fault-path check without a fault: the number of polls the stage kernels make on a tile's data
- * barrier before their bounded wait gives up (default and maximum 4,194,304; a negative value
- * restores the default).  With 0 every wait gives up at once: the kernel lets the copies it issued
- * land, marks the run failed and returns, the run stops after that stage with E3D_ERR_TIMEOUT, and
- * the handle stays usable.  Face-tile stage kernels only (the per-cell gather kernels never wait).
- * Kept for later runs of this solver, also inside a batch.  No counterpart in the reference, which
- * has no device waits. */
+/* Fault-path check without a fault: the number of polls that a kernel makes in a bounded wait before it
+ * gives up (default and maximum 4,194,304; a negative value restores the default).  The waits are those
+ * of the face-tile kernels for a tile's data and, in the resident kernel, also those of its blocks for one
+ * another.  With 0 every wait gives up at once: the kernel lets the copies it issued land, marks the run
+ * failed and returns, the run stops with E3D_ERR_TIMEOUT, and the handle stays usable.  With a small
+ * limit a resident run may give up after some of its tiles have gone on; the state is then that of no
+ * iteration and is to be loaded again.  The per-cell gather kernels never wait.  Kept for later runs of
+ * this solver, also inside a batch.  No counterpart in the reference, which has no device waits. */
 e3d_status e3d_solver_set_wait_limit(e3d_solver *solver, int32_t polls);
 
 /* Accuracy check of the FP64 mode's fast reciprocal and reciprocal square root (the hardware's coarse
