@@ -219,37 +219,33 @@ struct Batch {
         else if (precision == E3D_PREC_FP64_EXACT) prepare_batch_exact(smem, wss);
         else prepare_batch_fast(smem, wss);
         static const double alphas[5] = {0.0533, 0.1263, 0.2375, 0.4414, 1.0};
-        cudaGraph_t g;
-        E3D_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < iters; i++) {
-            const int p = i & 1;
-            for (int s = 0; s < 5; s++) {
-                BatchStage bs{};
-                bs.args = args.p;
-                bs.table = table.p;
-                bs.n_entries = counts.p;
-                bs.alpha = alphas[s];
-                bs.first_stage = s == 0;
-                bs.last_stage = s == 4;
-                bs.parity = p ^ (s & 1);
-                if (s == 0 && !apart) {
-                    bs.force_blocks = kBatchForceBlocks * member_cap;
-                    bs.n_members = counts.p + 1;
-                    bs.cargs = cargs.p;
+        graph = capture_graph(stream, [&] {
+            for (int i = 0; i < iters; i++) {
+                const int p = i & 1;
+                for (int s = 0; s < 5; s++) {
+                    BatchStage bs{};
+                    bs.args = args.p;
+                    bs.table = table.p;
+                    bs.n_entries = counts.p;
+                    bs.alpha = alphas[s];
+                    bs.first_stage = s == 0;
+                    bs.last_stage = s == 4;
+                    bs.parity = p ^ (s & 1);
+                    if (s == 0 && !apart) {
+                        bs.force_blocks = kBatchForceBlocks * member_cap;
+                        bs.n_members = counts.p + 1;
+                        bs.cargs = cargs.p;
+                    }
+                    launch_stage(bs);
                 }
-                launch_stage(bs);
+                launch_finalize_batch(fargs.p, counts.p + 1, member_cap, precision == E3D_PREC_FP64_EXACT, stream);
+                if (apart) launch_coeff_batch(cargs.p, counts.p + 1, 1 - p, member_cap, stream);
             }
-            launch_finalize_batch(fargs.p, counts.p + 1, member_cap, precision == E3D_PREC_FP64_EXACT, stream);
-            if (apart) launch_coeff_batch(cargs.p, counts.p + 1, 1 - p, member_cap, stream);
-        }
-        if (!apart) launch_coeff_batch(cargs.p, counts.p + 1, 0, member_cap, stream);  // the last iteration's
-        launch_control_gather(ctlp.p, counts.p + 1, ctl_all.p, member_cap, stream);
-        cudaMemcpyAsync(ctl_host, ctl_all.p, (size_t)member_cap * sizeof(Control), cudaMemcpyDeviceToHost, stream);
-        cudaError_t cap = cudaStreamEndCapture(stream, &g);
-        E3D_CUDA(cap);
-        cudaError_t inst = cudaGraphInstantiate(&graph, g, 0);
-        cudaGraphDestroy(g);
-        E3D_CUDA(inst);
+            if (!apart) launch_coeff_batch(cargs.p, counts.p + 1, 0, member_cap, stream);  // the last iteration's
+            launch_control_gather(ctlp.p, counts.p + 1, ctl_all.p, member_cap, stream);
+            E3D_CUDA(cudaMemcpyAsync(ctl_host, ctl_all.p, (size_t)member_cap * sizeof(Control), cudaMemcpyDeviceToHost,
+                                     stream));
+        });
         graph_iters = iters;
         graph_apart = apart;
         graph_builds++;

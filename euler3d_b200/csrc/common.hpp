@@ -62,6 +62,30 @@ void launch_dependent(void (*kernel)(Params...), int grid, int block, size_t sme
     E3D_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
 }
 
+// What `body` queues on the stream, as a graph.  The capture ends however body does: it may throw (a launch
+// that fails), and the stream may be the caller's own.
+template <typename F>
+cudaGraphExec_t capture_graph(cudaStream_t s, F &&body) {
+    struct Graph {
+        cudaGraph_t g = nullptr;
+        ~Graph() {
+            if (g) cudaGraphDestroy(g);
+        }
+    } graph;
+    E3D_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    try {
+        body();
+    } catch (...) {
+        cudaStreamEndCapture(s, &graph.g);
+        cudaGetLastError();
+        throw;
+    }
+    E3D_CUDA(cudaStreamEndCapture(s, &graph.g));
+    cudaGraphExec_t exec = nullptr;
+    E3D_CUDA(cudaGraphInstantiate(&exec, graph.g, 0));
+    return exec;
+}
+
 // Runs fn and converts exceptions into an e3d_status plus the thread's last-error message.
 template <typename F>
 e3d_status guarded(F &&fn) {

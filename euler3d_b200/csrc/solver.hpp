@@ -579,19 +579,14 @@ struct Solver {
             E3D_CUDA(cudaEventCreate(&e));
             graph_ev.push_back(e);
         }
-        cudaGraph_t g;
-        E3D_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        int b = 0;
-        for (int i = 0; i < iters; i++) {
-            enqueue_iteration(b, timed ? graph_ev.data() + 2 * (size_t)n_stages() * i : nullptr, defer);
-            b = 1 - b;  // five stages flip the buffer once per iteration
-        }
-        if (defer) enqueue_forces(b);
-        cudaError_t cap = cudaStreamEndCapture(stream, &g);
-        E3D_CUDA(cap);
-        cudaError_t inst = cudaGraphInstantiate(&graph, g, 0);
-        cudaGraphDestroy(g);
-        E3D_CUDA(inst);
+        graph = capture_graph(stream, [&] {
+            int b = 0;
+            for (int i = 0; i < iters; i++) {
+                enqueue_iteration(b, timed ? graph_ev.data() + 2 * (size_t)n_stages() * i : nullptr, defer);
+                b = 1 - b;  // five stages flip the buffer once per iteration
+            }
+            if (defer) enqueue_forces(b);
+        });
         graph_iters = iters;
         graph_timed = timed;
         graph_defer = defer;
