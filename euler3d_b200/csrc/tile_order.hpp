@@ -122,10 +122,14 @@ struct TileBisector {
                 for (int q = 0; q < nd; q++) cost[q] += std::fabs(d[0] * dir[q][0] + d[1] * dir[q][1] + d[2] * dir[q][2]);
             }
         }
+        // no plane cuts across a direction in which the part is flat but for rounding: a mesh one layer thick
+        // has one, whose cost of almost nothing over almost nothing would rank anywhere
+        double size = 1e-300;
+        for (int q = 0; q < nd; q++) size = std::max({size, std::fabs(lo[q]), std::fabs(hi[q]), hi[q] - lo[q]});
         int rank[kDirs];
         for (int q = 0; q < nd; q++) {
             rank[q] = q;
-            cost[q] /= std::max(hi[q] - lo[q], 1e-300);
+            cost[q] = hi[q] - lo[q] > 1e-13 * size ? cost[q] / (hi[q] - lo[q]) : HUGE_VAL;
         }
         int tries = std::min(nd, coarse ? 1 : n > 16 * tile ? 2 : 4);
         std::partial_sort(rank, rank + tries, rank + nd,
