@@ -1098,6 +1098,48 @@ void begin_run(Solver *S, const e3d_run_params *rp, bool defer, cudaStream_t s) 
     S->records_valid = true;
 }
 
+// Blocks that wait for one another need the whole grid on the GPU: one resident kernel per device at a time
+// in this process.  Not locked: none is possible, or another solver has it (a run takes the stage kernels
+// then, with the same results).
+static std::unique_lock<std::mutex> lock_resident(Solver *S) {
+    static std::mutex busy[64];
+    if (S->device >= 64 || !S->resident_ready()) return {};
+    return std::unique_lock<std::mutex>(busy[S->device], std::try_to_lock);
+}
+
+// Where more tiles share an SM than the resident kernel is always the faster one for (kTimedShape): times
+// some iterations from the freestream both ways, each once to warm up, and gives the kernel up if it
+// loses.  Leaves the solver as it was made.
+static void tune_resident(Solver *S) {
+    constexpr int kIterations = 12;
+    if (!S->resident_ready() || S->resident_shape < kTimedShape) return;
+    const std::unique_lock<std::mutex> lock = lock_resident(S);
+    if (!lock.owns_lock()) return;
+    e3d_run_params rp{};
+    rp.max_iter = 2 * kIterations;  // no stop
+    rp.sampling = 1;
+    float ms[2] = {0.f, 0.f};
+    for (int k = 0; k < 4; k++) {
+        const bool resident = k & 1, defer = !resident && S->can_defer();
+        begin_run(S, &rp, defer, S->stream);
+        E3D_CUDA(cudaEventRecord(S->ev0, S->stream));
+        if (resident) {
+            if (!S->launch_resident(kIterations)) break;
+        } else {
+            for (int i = 0; i < kIterations; i++) S->enqueue_iteration(i & 1, nullptr, defer);
+            if (defer) S->enqueue_forces(0);
+            E3D_CUDA(cudaGetLastError());
+        }
+        E3D_CUDA(cudaEventRecord(S->ev1, S->stream));
+        E3D_CUDA(cudaEventSynchronize(S->ev1));
+        E3D_CUDA(cudaEventElapsedTime(&ms[resident], S->ev0, S->ev1));
+    }
+    if (ms[0] < ms[1]) S->resident_shape = -1;
+    if (S->resident_shape < 0) S->release_resident();
+    if (S->n_wall) E3D_CUDA(cudaMemsetAsync(S->wall_cp.p, 0, S->n_wall * sizeof(double), S->stream));
+    set_freestream(S);
+}
+
 void stats_from_control(const Control &c, e3d_run_stats *st) {
     st->iterations = c.it;
     st->stop_reason = c.stop_reason;
@@ -1130,8 +1172,12 @@ e3d_status e3d_solver_create(const e3d_mesh_desc *mesh, const e3d_flow_params *p
     e3d_status st = guarded([&] {
         create_solver(mesh, params, S.get());
         set_freestream(S.get());
-        if (params->no_autotune) S->use_default_variant();
-        else S->autotune();
+        if (params->no_autotune) {
+            S->use_default_variant();
+        } else {
+            S->autotune();
+            tune_resident(S.get());
+        }
     });
     if (st == E3D_OK) *out = reinterpret_cast<e3d_solver *>(S.release());
     return st;
@@ -1261,12 +1307,8 @@ e3d_status e3d_solver_run(e3d_solver *solver, const e3d_run_params *rp, e3d_run_
         double stage_ms = 0.0;
         int64_t stage_launches = 0;
         if (rp->profile_stages < 0 || rp->profile_stages > 2) throw Error(E3D_ERR_INVALID_ARG, "profile_stages must be 0, 1 or 2");
-        // Blocks that wait for one another need the whole grid on the GPU: one resident run per device
-        // at a time in this process (a run beside it takes the stage kernels, with the same results).
-        static std::mutex resident_busy[64];
         std::unique_lock<std::mutex> resident;
-        if (rp->profile_stages == 0 && !S->variant_forced && S->device < 64 && S->resident_ready())
-            resident = std::unique_lock<std::mutex>(resident_busy[S->device], std::try_to_lock);
+        if (rp->profile_stages == 0 && !S->variant_forced) resident = lock_resident(S);
         // Forces that cannot stop the run are left to the next iteration's first stage (the resident
         // kernel's control block has its own way, and timed stages hold nothing else).
         const bool defer = !resident.owns_lock() && rp->profile_stages == 0 && S->can_defer() && !forces_decide(rp);

@@ -180,8 +180,7 @@ struct Solver {
         tile_rec32_off.release();
         tile_contrib.release();
         release_colours();
-        resident_flags.release();
-        resident_words.release();
+        release_resident();
         cf.release();
         fgeo.release();
         cgeo.release();
@@ -335,6 +334,12 @@ struct Solver {
         }
         E3D_CUDA(cudaMemsetAsync(resident_words.p, 0, resident_words.n * sizeof(uint4), stream));
         return true;
+    }
+
+    void release_resident() {
+        resident_flags.release();
+        resident_words.release();
+        resident_flags.n = resident_words.n = 0;
     }
 
     // `iters` iterations from state buffer 0 with the resident kernel; false (and never again): they do

@@ -449,6 +449,19 @@ struct ResidentShape {
 constexpr ResidentShape kResidentShapes[] = {{512, 1}, {256, 2}, {256, 3}, {128, 4}, {128, 6}};
 constexpr int kResidentShapeCount = 5;
 
+// The more tiles share an SM, the less the stage kernels' fixed costs weigh.  us per RK5 iteration, forces
+// sampled every iteration, autotuned stage kernels against this kernel (B200):
+//   tiles        channel, 2 layers       O-grid, 4 layers        box of tetrahedra
+//   FP64         436  45.0  31.6         436  43.7  34.9         435  42.8  35.6
+//                587  46.6  41.5         587  44.8  49.2         571  44.0  48.4      648  55.1  62.6
+//   FP32_FLUX    587  47.4  36.4         587  43.8  37.4         571  42.2  43.9      648  42.2  48.4
+//                704  47.3  47.7         781  44.4  57.6         824  43.8  57.5
+//   FP64_EXACT   291   126   111         313   152   207         289   127   118      375   143   225
+// Up to three tiles per SM (two in exact mode, whose RMS and forces are the control block's sequential
+// sums) it is the faster one everywhere; with more, the shapes of 128 threads, that depends on the mesh, and
+// the creation of a tuned solver times both ways.
+constexpr int kTimedShape = 3;
+
 template <int PREC>
 struct ResidentLaunch {
     static const void *kernel(int shape) {

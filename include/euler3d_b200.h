@@ -215,7 +215,8 @@ typedef struct e3d_run_params {
 	                                     so the stages are timed as they run back to back
 	                                     (stats.stage_ms over the iterations that ran) */
 	int32_t stage_kernel;             /* 0: the resident kernel (whole iterations in one launch) where the
-	                                     mesh's face tiles all fit on the GPU at once, otherwise the
+	                                     mesh's face tiles all fit on the GPU at once (and, beyond three
+	                                     per SM, the tuning found it faster), otherwise the
 	                                     autotuned stage kernel; 1, 2: per-cell gather with two
 	                                     register budgets (FP64 modes); 3: face tiles; 4: persistent
 	                                     face tiles with a producer warp streaming tiles to consumer
