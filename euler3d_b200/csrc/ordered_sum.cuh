@@ -28,9 +28,6 @@ struct OrderedScratch {
     long long prefix[kSpecials];  // whole units before a special element
     double value[kSpecials];
     int expo[kSpecials];          // binade of the sum before it
-    long long units;              // whole units of all elements
-    double sum;
-    int fail;
 };
 
 __device__ __forceinline__ int biased_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
@@ -147,7 +144,6 @@ __device__ double ordered_sum(const double *x, int n, OrderedScratch &sh, double
     const int slot = block_scan<NT>(count, sh.warp_count, n_special);
     long long all_units;
     const long long units_before = block_scan<NT>(units, sh.warp_units, all_units);
-    if (tid == 0) sh.fail = 0;
     bad = __syncthreads_or(bad) || n_special > kSpecials;
     if (!bad && count) {
         int k = slot;
