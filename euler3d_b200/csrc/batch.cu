@@ -61,6 +61,7 @@ struct Batch {
     int ws_buffers = 0;
     size_t ws_stride = 0, ws_smem = 0;
     int n_entries = 0;
+    bool many_faces = false;  // a member has cells of more than six faces: one kernel serves such batches
     bool dirty = true;
 
     cudaGraphExec_t graph = nullptr;
@@ -110,8 +111,10 @@ struct Batch {
         std::vector<Control *> P(nm);
         std::vector<int2> T;
         size_t smem = 0;
+        bool many = false;
         for (int m = 0; m < nm; m++) {
             Solver *S = members[m].S;
+            many |= S->max_contrib > kElementFaces;
             for (int b = 0; b < 2; b++) {
                 A[2 * m + b] = S->stage_args(b, 0.0, 0, 0);  // alpha and stage flags come per launch
                 C[2 * m + b] = S->coeff_args(b, 1, nullptr);
@@ -153,6 +156,10 @@ struct Batch {
             drop_graph();
             smem_cap = smem;
         }
+        if (many != many_faces) {
+            drop_graph();
+            many_faces = many;
+        }
         // the warp-specialised kernel's buffers: the largest member's tile data plus its arguments
         size_t stride = 0;
         for (const Member &m : members) {
@@ -181,7 +188,7 @@ struct Batch {
         dirty = false;
     }
 
-    bool use_ws() const { return kernel == E3D_BATCH_KERNEL_WS && ws_buffers >= 2; }
+    bool use_ws() const { return kernel == E3D_BATCH_KERNEL_WS && ws_buffers >= 2 && !many_faces; }
 
     // Force coefficients in a kernel of their own after every iteration: a member's may stop its run, or
     // the stage kernel has no force blocks.  Otherwise the next first stage integrates them.
@@ -204,9 +211,9 @@ struct Batch {
         }
         const int grid = tile_cap + bs.force_blocks;
         const size_t smem = with_forces(smem_cap, bs.force_blocks);
-        if (precision == E3D_PREC_FP32_FLUX) launch_batch_f32(bs, grid, smem, stream);
-        else if (precision == E3D_PREC_FP64_EXACT) launch_batch_exact(bs, grid, smem, stream);
-        else launch_batch_fast(bs, grid, smem, stream);
+        if (precision == E3D_PREC_FP32_FLUX) launch_batch_f32(bs, many_faces, grid, smem, stream);
+        else if (precision == E3D_PREC_FP64_EXACT) launch_batch_exact(bs, many_faces, grid, smem, stream);
+        else launch_batch_fast(bs, many_faces, grid, smem, stream);
     }
 
     // `iters` iterations (even, so every running member ends on state buffer 0) + the control

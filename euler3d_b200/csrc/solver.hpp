@@ -43,9 +43,9 @@ void launch_update_fast(const StageArgs &a, cudaStream_t s);
 void prepare_batch_exact(size_t smem_bytes, size_t ws_smem_bytes);
 void prepare_batch_fast(size_t smem_bytes, size_t ws_smem_bytes);
 void prepare_batch_f32(size_t smem_bytes, size_t ws_smem_bytes);
-void launch_batch_exact(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
-void launch_batch_fast(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
-void launch_batch_f32(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
+void launch_batch_exact(const BatchStage &bs, bool many_faces, int grid, size_t smem_bytes, cudaStream_t s);
+void launch_batch_fast(const BatchStage &bs, bool many_faces, int grid, size_t smem_bytes, cudaStream_t s);
+void launch_batch_f32(const BatchStage &bs, bool many_faces, int grid, size_t smem_bytes, cudaStream_t s);
 void launch_batch_ws_exact(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
 void launch_batch_ws_fast(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
 void launch_batch_ws_f32(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s);
@@ -298,7 +298,7 @@ struct Solver {
     // that the solver's stream may use.
     void plan_resident() {
         resident_planned = true;
-        if (!tiles_ok || smoothing) return;
+        if (!tiles_ok || smoothing || max_contrib > kElementFaces) return;
         const int prec = f32 ? PREC_F32 : prm.precision == E3D_PREC_FP64 ? PREC_FAST : PREC_EXACT;
         size_t smem = resident_smem_bytes(prec, smem_cells, smem_faces, max_contrib, max_far, n_tiles);
         const int sms = stream_sms(stream, n_sm);

@@ -35,6 +35,7 @@ constexpr int kStageThreads = 128;
 constexpr int kTileCells = kStageThreads;   // cells owned by one face tile (one per thread)
 constexpr int kTileLocalBits = 10;          // local (owned + halo) cell index in a tile face entry
 constexpr unsigned short kNoContrib = 0xFFFF;
+constexpr int kElementFaces = 6;  // faces of the element type that has most
 
 struct Freestream {
     double rho, u, v, w, p, E, H, M;
@@ -1083,19 +1084,22 @@ __device__ __forceinline__ void tile_load_cell(const StageArgs &a, int c0, int i
 
 // Cell i of the tile: sum of its contributions, then time step and update; returns R_rho^2 on
 // the last stage.  W0 and the geometry come from the caller, which loads them before the barrier
-// that ends the flux phase so that their latency overlaps the wait.
-template <bool EXACT, typename STEP>
+// that ends the flux phase so that their latency overlaps the wait.  MANY: cells of more faces than the
+// element types have.  Its loop stands between the sums and the time step, which otherwise overlap: in the
+// kernels of ordinary meshes it cost 1 to 2 % (4,096-cell channel, 200 iterations in the resident kernel
+// 3.55 -> 3.59 ms; FP32_FLUX batch of 16 members 16.6 -> 16.9), so only kernels of their own have it.
+template <bool EXACT, bool MANY = false, typename STEP>
 __device__ __forceinline__ double tile_update(const StageArgs &a, const STEP &sp, const TileBuf &b,
                                               const double *fs, int c0, int i, double W0[5], const double4 &cg,
                                               Prim &out) {
     const int T = kTileCells;
     double R[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    unsigned short e[6];
+    unsigned short e[kElementFaces];
 #pragma unroll
-    for (int k = 0; k < 6; k++) e[k] = k < a.max_contrib ? b.ct[k * T + i] : kNoContrib;
+    for (int k = 0; k < kElementFaces; k++) e[k] = k < a.max_contrib ? b.ct[k * T + i] : kNoContrib;
     const Prim me = tile_prim(b.st, i);
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
+    for (int k = 0; k < kElementFaces; k++) {
         if (e[k] == kNoContrib) break;
         const int j = e[k] >> 1;
         // R -/+ F*S as one fused multiply-add by -/+1: the product is exact and the sum rounds once,
@@ -1104,7 +1108,7 @@ __device__ __forceinline__ double tile_update(const StageArgs &a, const STEP &sp
 #pragma unroll
         for (int q = 0; q < 5; q++) R[q] = fma(sg, fs[5 * j + q], R[q]);
     }
-    for (int k = 6; k < a.max_contrib; k++) {  // cells of more faces than the element types have
+    for (int k = kElementFaces; MANY && k < a.max_contrib; k++) {
         const unsigned x = b.ct[k * T + i];
         if (x == kNoContrib) break;
         const double sg = (x & 1) ? -1.0 : 1.0;
@@ -1141,7 +1145,7 @@ __device__ __forceinline__ bool run_stopped(const StageArgs &a) {
 // Shared memory: TileBuf (face fluxes over the records) | mbarrier
 // The body is shared by tile_kernel (one solver) and tile_batch_kernel (several solvers in one
 // grid): `tile` is the solver's own tile index, `partial` where its RMS partial goes.
-template <bool EXACT>
+template <bool EXACT, bool MANY>
 __device__ __forceinline__ void tile_body(const StageArgs &a, int tile, double *partial, unsigned char *smem_raw) {
     const int LC = a.smem_cells, FC = a.smem_faces, MC = a.max_contrib, T = kTileCells;
     const TileBuf b = tile_buf_at(smem_raw, LC, FC, MC);
@@ -1203,11 +1207,11 @@ __device__ __forceinline__ void tile_body(const StageArgs &a, int tile, double *
     __syncthreads();
     double r2 = 0.0;
     Prim out;
-    if ((int)threadIdx.x < nloc) r2 = tile_update<EXACT>(a, sp, b, fs, c0, threadIdx.x, W0, cg, out);
+    if ((int)threadIdx.x < nloc) r2 = tile_update<EXACT, MANY>(a, sp, b, fs, c0, threadIdx.x, W0, cg, out);
     if (a.last_stage && !a.residual_only) block_sum_store(r2, partial);
 }
 
-template <bool EXACT, int MINB>
+template <bool EXACT, int MINB, bool MANY = false>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel(StageArgs a, const __grid_constant__ CoeffArgs c) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     pdl_release();
@@ -1217,7 +1221,7 @@ __global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel(StageArgs a, 
         force_block(c, blockIdx.x, a.force_blocks, smem_raw);
         return;
     }
-    tile_body<EXACT>(a, tile, a.partials + tile, smem_raw);
+    tile_body<EXACT, MANY>(a, tile, a.partials + tile, smem_raw);
 }
 
 // ---- several solvers ("members") in one grid
@@ -1277,7 +1281,7 @@ __device__ __forceinline__ int batch_entry(const BatchStage &bs, unsigned char *
     return -1;
 }
 
-template <bool EXACT, int MINB>
+template <bool EXACT, int MINB, bool MANY = false>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel(BatchStage bs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     pdl_release();
@@ -1285,7 +1289,7 @@ __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel(BatchSt
     if (entry < 0) return;  // uniform across the block
     __shared__ __align__(16) StageArgs sa;
     const int2 e = batch_stage_args(bs, entry, &sa);
-    tile_body<EXACT>(sa, e.y, sa.partials + e.y, smem_raw);
+    tile_body<EXACT, MANY>(sa, e.y, sa.partials + e.y, smem_raw);
 }
 
 // ---- update phase of a split stage

@@ -193,7 +193,8 @@ __device__ __forceinline__ void tile_load_cell_f32(const StageArgs &a, int c, do
 }
 
 // Cell i of the tile: sum of its faces' F*S, time step and update; returns R_rho^2 on the last stage.
-template <typename STEP>
+// MANY: as for tile_update.
+template <bool MANY = false, typename STEP>
 __device__ __forceinline__ double tile_update_f32(const StageArgs &a, const STEP &sp, const Tile32 &b,
                                                   const float *fs, int c0, int i, double W0[5], const float4 &cg,
                                                   PrimF &out) {
@@ -201,18 +202,18 @@ __device__ __forceinline__ double tile_update_f32(const StageArgs &a, const STEP
     const float gf = (float)a.gamma;
     const PrimF me = prim32(b.st, i);
     double R[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    unsigned short e[6];
+    unsigned short e[kElementFaces];
 #pragma unroll
-    for (int k = 0; k < 6; k++) e[k] = k < MC ? b.ct[k * T + i] : kNoContrib;
+    for (int k = 0; k < kElementFaces; k++) e[k] = k < MC ? b.ct[k * T + i] : kNoContrib;
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
+    for (int k = 0; k < kElementFaces; k++) {
         if (e[k] == kNoContrib) break;
         const int j = e[k] >> 1;
         const double sg = (e[k] & 1) ? -1.0 : 1.0;  // fma by -/+1: the bits of R -/+ F*S (see tile_update)
 #pragma unroll
         for (int q = 0; q < 5; q++) R[q] = fma(sg, (double)fs[6 * j + q], R[q]);
     }
-    for (int k = 6; k < MC; k++) {  // cells of more faces than the element types have
+    for (int k = kElementFaces; MANY && k < MC; k++) {
         const unsigned x = b.ct[k * T + i];
         if (x == kNoContrib) break;
         const double sg = (x & 1) ? -1.0 : 1.0;
@@ -255,6 +256,7 @@ __device__ __forceinline__ double tile_update_f32(const StageArgs &a, const STEP
 
 // Body shared by tile_kernel_f32 (one solver) and tile_batch_kernel_f32 (several solvers in one
 // grid): `tile` is the solver's own tile index, `partial` where its RMS partial goes.
+template <bool MANY>
 __device__ __forceinline__ void tile_body_f32(const StageArgs &a, int tile, double *partial, unsigned char *smem_raw) {
     const int LC = a.smem_cells, FC = a.smem_faces, MC = a.max_contrib, T = kTileCells;
     const Tile32 b = tile32_at(smem_raw, LC, FC);
@@ -325,11 +327,11 @@ __device__ __forceinline__ void tile_body_f32(const StageArgs &a, int tile, doub
     __syncthreads();
     double r2 = 0.0;
     PrimF out;
-    if (i < nloc) r2 = tile_update_f32(a, sp, b, fs, c0, i, W0, cg, out);
+    if (i < nloc) r2 = tile_update_f32<MANY>(a, sp, b, fs, c0, i, W0, cg, out);
     if (a.last_stage && !a.residual_only) block_sum_store(r2, partial);
 }
 
-template <int MINB>
+template <int MINB, bool MANY = false>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel_f32(StageArgs a,
                                                                        const __grid_constant__ CoeffArgs c) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -340,11 +342,11 @@ __global__ void __launch_bounds__(kStageThreads, MINB) tile_kernel_f32(StageArgs
         force_block(c, blockIdx.x, a.force_blocks, smem_raw);
         return;
     }
-    tile_body_f32(a, tile, a.partials + tile, smem_raw);
+    tile_body_f32<MANY>(a, tile, a.partials + tile, smem_raw);
 }
 
 // Several solvers in one grid (see tile_batch_kernel).
-template <int MINB>
+template <int MINB, bool MANY = false>
 __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel_f32(BatchStage bs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     pdl_release();
@@ -352,7 +354,7 @@ __global__ void __launch_bounds__(kStageThreads, MINB) tile_batch_kernel_f32(Bat
     if (entry < 0) return;
     __shared__ __align__(16) StageArgs sa;
     const int2 e = batch_stage_args(bs, entry, &sa);
-    tile_body_f32(sa, e.y, sa.partials + e.y, smem_raw);
+    tile_body_f32<MANY>(sa, e.y, sa.partials + e.y, smem_raw);
 }
 
 }  // namespace e3d

@@ -9,11 +9,13 @@ namespace e3d {
 void prepare_tile_fast(size_t smem_bytes, size_t pipe_smem_bytes) {
     raise_smem_limit((const void *)tile_kernel<false, 4>, with_forces(smem_bytes, 1));
     raise_smem_limit((const void *)tile_kernel<false, 7>, with_forces(smem_bytes, 1));
+    raise_smem_limit((const void *)tile_kernel<false, 4, true>, with_forces(smem_bytes, 1));
     if (pipe_smem_bytes) raise_smem_limit((const void *)tile_ws_kernel<WS_FAST>, pipe_smem_bytes);
 }
 
 void prepare_batch_fast(size_t smem_bytes, size_t ws_smem_bytes) {
     raise_smem_limit((const void *)tile_batch_kernel<false, 6>, smem_bytes);
+    raise_smem_limit((const void *)tile_batch_kernel<false, 4, true>, smem_bytes);
     if (ws_smem_bytes) raise_smem_limit((const void *)tile_ws_batch_kernel<WS_FAST>, ws_smem_bytes);
 }
 
@@ -23,8 +25,9 @@ void launch_update_fast(const StageArgs &a, cudaStream_t s) {
 }
 
 // One stage of every member of a batch: `grid` blocks over the (member, tile) table.
-void launch_batch_fast(const BatchStage &bs, int grid, size_t smem_bytes, cudaStream_t s) {
-    launch_dependent(tile_batch_kernel<false, 6>, grid, kStageThreads, smem_bytes, s, bs);
+void launch_batch_fast(const BatchStage &bs, bool many_faces, int grid, size_t smem_bytes, cudaStream_t s) {
+    launch_dependent(many_faces ? tile_batch_kernel<false, 4, true> : tile_batch_kernel<false, 6>, grid, kStageThreads,
+                     smem_bytes, s, bs);
 }
 
 // The same stage with the warp-specialised persistent kernel: `grid` blocks walk the table.
@@ -64,10 +67,14 @@ void launch_colour_finish_fast(const StageArgs &a, const double2 *rc, cudaStream
 
 // variant 0: gather kernel, registers for 4 blocks/SM; 1: gather kernel, 5 blocks/SM;
 // 2: face tiles, one block per tile (4 blocks/SM); 3: face tiles, persistent and warp-specialised;
-// 4: face tiles with registers for 7 blocks/SM
+// 4: face tiles with registers for 7 blocks/SM.  Meshes with cells of more than six faces have one
+// face-tile kernel.
 void launch_stage_fast(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant) {
     const int blocks = (a.n_cells + kStageThreads - 1) / kStageThreads;
-    if (variant == 4) {
+    if (variant >= 2 && a.max_contrib > kElementFaces) {
+        const size_t smem = with_forces(tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib), a.force_blocks);
+        launch_dependent(tile_kernel<false, 4, true>, blocks + a.force_blocks, kStageThreads, smem, s, a, c);
+    } else if (variant == 4) {
         const size_t smem = tile_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
         launch_dependent(tile_kernel<false, 7>, blocks + a.force_blocks, kStageThreads, with_forces(smem, a.force_blocks), s, a, c);
     } else if (variant == 3) {

@@ -223,7 +223,8 @@ typedef struct e3d_run_params {
 	                                     warps; 5: face tiles at seven blocks per SM (FP64) or nine
 	                                     (FP32_FLUX); 6, 7: face colouring, one launch per class of
 	                                     faces that share no cell, 128 or 512 faces per block (FP64)
-	                                     (kept for later runs) */
+	                                     (kept for later runs).  On a mesh with cells of more than six
+	                                     faces 3, 4 and 5 are one kernel, and 0 is never the resident */
 	double min_residual_drop;         /* > 0: also stop once the density RMS is below this fraction of
 	                                     the run's first RMS (a relative tolerance such as 1e-8); 0 off.
 	                                     No counterpart in the reference, whose test is absolute. */
@@ -372,7 +373,8 @@ e3d_status e3d_batch_remove(e3d_batch *batch, e3d_solver *solver, e3d_run_stats 
  *   E3D_BATCH_KERNEL_WS     one persistent block per SM walking the table: a producer warp copies each
  *                           entry's member arguments and tile data into a ring of shared-memory buffers
  *                           ahead of five consumer groups that evaluate them
- * Both compute the same bits.  No counterpart in the reference. */
+ * Both compute the same bits; with a member whose mesh has cells of more than six faces the first is used.
+ * No counterpart in the reference. */
 enum { E3D_BATCH_KERNEL_TILES = 0, E3D_BATCH_KERNEL_WS = 1 };
 e3d_status e3d_batch_set_kernel(e3d_batch *batch, int32_t kernel);
 
