@@ -24,9 +24,11 @@
 // The arithmetic is that of the stage kernels (the same functions), so states, RMS history and
 // coefficients have the same bits.
 //
-// What bounds it is the chain of a stage in one tile: 0.8 us for the halo's trip through L2, 1.0 us for
-// the slowest face and 0.9 us for the update (FP64 latency and instruction issue of the few warps of
-// one tile), 0.5 us of waiting for slower neighbours.  Measured on B200, us per RK5 iteration with force
+// What bounds it is the chain of a stage in one tile, 3.55 us on a channel of 4,096 FP64 cells: 1.2 us
+// for the halo (0.6 its words' trip through L2, the rest waiting for slower neighbours; 1.7 before an
+// iteration's last stage, with the decision and the forces), 0.9 us for the fluxes and 1.2 us for the
+// update (FP64 latency and instruction issue of the few warps of one tile; the issue slots are 21 % used).
+// Measured on B200, us per RK5 iteration with force
 // sampling every iteration, CUDA graphs of stage kernels against this kernel:
 //   channel 4,096 cells FP64          55.8   17.1      O-grid 20,200 cells, AUSM, FP64      50.5   21.2
 //   channel 37,442 cells FP32_FLUX    52.2   20.5      channel 16,770 cells FP64_EXACT       506   42.7
