@@ -31,7 +31,8 @@ void launch_batch_f32(const BatchStage &bs, bool many_faces, int grid, size_t sm
 // variant 2: face tiles with registers for four blocks/SM; 3: warp-specialised persistent face
 // tiles; 4: face tiles at nine blocks/SM (56 registers, no spills; 1.57M tetrahedra 71.7 us a stage at
 // eight blocks, 69.5 at nine, 561k-cell AUSM channel 25.0 and 23.4; the batch kernel spills at nine and
-// takes 141 us an iteration instead of 131, so it stays at eight)
+// takes 141 us an iteration instead of 131, so it stays at eight; an iteration's first stage runs at eight
+// too where it carries force blocks, whose 24 KB are more than a tile's 17.8)
 void launch_stage_f32(const StageArgs &a, const CoeffArgs &c, cudaStream_t s, int variant) {
     const int blocks = (a.n_cells + kStageThreads - 1) / kStageThreads;
     const size_t smem = tile32_smem_bytes(a.smem_cells, a.smem_faces, a.max_contrib);
