@@ -370,19 +370,26 @@ __device__ __forceinline__ void ausm_fast(const Prim &L, const Prim &R, double r
     ausm_tail(L, R, cl, cr, Vl, Vr, Vl * (L.rho * rl), Vr * (R.rho * rr), nx, ny, nz, F);
 }
 
-// Fast: the flux through a symmetry face, between cell state d and its mirror image (the same density,
-// pressure and enthalpy, the normal velocity reversed).  The mirror symmetry leaves a normal force
-// only: mass, energy and tangential terms cancel.
+// Total enthalpy of the mirror image; out of line, since only the first stage of a loaded state needs it.
+static __device__ __noinline__ double mirror_enthalpy(double p, double rho, double q2, double g) {
+    return fma(g, p * rcp_nr((g - 1.0) * rho), 0.5 * q2);
+}
+
+// Fast: the flux through a symmetry face, between cell state d and its mirror image (the same density and
+// pressure, the normal velocity reversed).  The mirror symmetry leaves a normal force only: mass, energy
+// and tangential terms cancel.
 //   Roe: the averages are the cell's tangential flow, V~ = 0, c~^2 = (gamma - 1)(H - q_t^2 / 2) with
 //     q_t^2 the tangential speed squared, both acoustic waves move at c~ >= c (the entropy fix never
 //     applies), and the force is p + rho V (V + c~).
 //   AUSM: the split Mach numbers cancel and the two split pressures are equal, force 2 p P+(V / c).
 // About 30 operations for the general flux's 200, and no ghost enthalpy (two divisions): on the
 // 2-layer channels every cell has a symmetry face.
+// A loaded state brings an H of its own, and the ghost's follows from p, rho and the velocity (`loaded`: no
+// stage has run since): H~ is their mean then, and half of rho V times their difference stays of the energy.
 __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double ny, double nz, double g, int scheme,
-                                              double F[5]) {
+                                              bool loaded, double F[5]) {
     const double V = fma(d.u, nx, fma(d.v, ny, d.w * nz));
-    double f;
+    double f, energy = 0.0;
     if (scheme == 1) {
         const double M = V * (d.rho * rsqrt_nr(g * d.p * d.rho));
         double pp;
@@ -390,15 +397,21 @@ __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double n
         else pp = M > 0.0 ? 1.0 : 0.0;
         f = 2.0 * pp * d.p;
     } else {
-        const double qt2 = fma(-V, V, fma(d.u, d.u, fma(d.v, d.v, d.w * d.w)));
-        const double c2 = (g - 1.0) * fma(-0.5, qt2, d.H);
+        double qt2 = fma(d.u, d.u, fma(d.v, d.v, d.w * d.w)), h = d.H;
+        if (loaded) {
+            const double hg = mirror_enthalpy(d.p, d.rho, qt2, g);
+            h = 0.5 * (d.H + hg);
+            energy = 0.5 * (d.rho * V) * (d.H - hg);
+        }
+        qt2 = fma(-V, V, qt2);
+        const double c2 = (g - 1.0) * fma(-0.5, qt2, h);
         f = fma(d.rho * V, V + c2 * rsqrt_nr(sign_or(c2, d.rho)), d.p);  // NaN for a negative density
     }
     F[0] = 0.0;
     F[1] = f * nx;
     F[2] = f * ny;
     F[3] = f * nz;
-    F[4] = 0.0;
+    F[4] = energy;
 }
 
 // ------------------------------------------------------------------------------ ghost states
@@ -599,7 +612,7 @@ __device__ __forceinline__ bool boundary_face(const StageArgs &a, const STEP &sp
     if (tag == TAG_SYM) {
         ghost_mirror<PREC>(gp, g, me, fg.x, fg.y, fg.z, gs, store, PREC != PREC_FAST);
         if (PREC != PREC_FAST) return true;
-        sym_flux_fast(me, fg.x, fg.y, fg.z, g, a.scheme, F);
+        sym_flux_fast(me, fg.x, fg.y, fg.z, g, a.scheme, sp.first_stage() && sp.minit_valid(), F);
         return false;
     }
     if (tag == TAG_FAR) {
