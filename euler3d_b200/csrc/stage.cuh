@@ -395,7 +395,8 @@ __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double n
         double pp;
         if (fabs(M) <= 1.0) pp = 0.25 * (M + 1.0) * (M + 1.0) * (2.0 - M);
         else pp = M > 0.0 ? 1.0 : 0.0;
-        f = 2.0 * pp * d.p;
+        f = fma(0.0, V, 2.0 * pp * d.p);  // NaN where V is no finite number, as the general flux's products
+        energy = 0.0 * (d.rho * V * d.H);
     } else {
         double qt2 = fma(d.u, d.u, fma(d.v, d.v, d.w * d.w)), h = d.H;
         if (loaded) {

@@ -101,3 +101,20 @@ def test_ghost_mach_of_a_fluid_at_rest(precision):
         s.residual()
         assert np.isnan(s.get_state()["M"][1:]).all()
         s.close()
+
+
+@pytest.mark.parametrize("kernel", DOUBLE_KERNELS)
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("key", ["u", "v", "w", "H"])
+def test_ausm_symmetry_faces_pass_on_nan(key, value, kernel):
+    """A velocity or an enthalpy that is no finite number: the symmetry faces of its cell, whose splits
+    cancel, still end in NaN where the reference's products do (0 x NaN, 0 x inf)."""
+    arrays = cube()
+    out = []
+    for prec, k in ((_lib.PREC_FP64_EXACT, _lib.KERNEL_TILE), (_lib.PREC_FP64, kernel)):
+        flow = FlowConfig(mach=0.5, cfl=1.0, precision=prec, scheme=_lib.SCHEME_AUSM)
+        state = perturbed_state(arrays, flow, 3)
+        state[key][0] = value
+        out.append(residual(arrays, flow, state, k)[0, 1:])
+    assert np.isnan(out[0]).any()
+    assert np.isnan(out[1])[np.isnan(out[0])].all()
