@@ -200,6 +200,16 @@ __device__ __forceinline__ double sign_or(double x, double y) {
     return __hiloint2double(__double2hiint(x) | (__double2hiint(y) & (int)0x80000000u), __double2loint(x));
 }
 
+// sqrt(a) sqrt(b) by one root, NaN where either is negative; outside the seed's range by two, since the
+// product may overflow or vanish where the roots do not (out of line: densities are not of that size).
+static __device__ __noinline__ double two_roots(double a, double b) { return sqrt(a) * sqrt(b); }
+
+__device__ __forceinline__ double root_of_product(double a, double b) {
+    const double x = sign_or(a * b, a);
+    if (!seed_ok(__double2hiint(x))) return two_roots(a, b);
+    return x * rsqrt_nr(x);
+}
+
 // ------------------------------------------------------------------------------ Roe flux
 // Exact: Solver::Roe (src/solver/ConvectiveFluxesSchemes.cpp:10-165) operation by operation.
 __device__ __forceinline__ void roe_exact(const Prim &L, const Prim &R, double nx, double ny, double nz,
@@ -269,8 +279,7 @@ __device__ __forceinline__ void roe_exact(const Prim &L, const Prim &R, double n
 // the same bits whatever its register budget.
 __device__ __forceinline__ void roe_fast(const Prim &L, const Prim &R, double nx, double ny, double nz, double g,
                                          double F[5]) {
-    const double rr = L.rho * R.rho;
-    const double rt = rr * rsqrt_nr(sign_or(rr, L.rho));  // NaN also where both densities are negative
+    const double rt = root_of_product(L.rho, R.rho);
     const double inv = rcp_nr(L.rho + rt);
     double wl = L.rho * inv, wr = rt * inv;
     double ut = fma(L.u, wl, R.u * wr);

@@ -118,3 +118,23 @@ def test_ausm_symmetry_faces_pass_on_nan(key, value, kernel):
         out.append(residual(arrays, flow, state, k)[0, 1:])
     assert np.isnan(out[0]).any()
     assert np.isnan(out[1])[np.isnan(out[0])].all()
+
+
+@pytest.mark.parametrize("kernel", DOUBLE_KERNELS)
+@pytest.mark.parametrize("power", [600, -600])
+def test_roe_of_densities_out_of_range(power, kernel):
+    """Densities and pressures whose products overflow or vanish although their roots do not: the fluxes are
+    proportional to them, so a power of two comes through, within the 2e-13 of test_gpu_fast_flux.py of the
+    sizes of a cell's face terms (at most eight times the largest component here)."""
+    arrays = prepared("tets")
+    flow = FlowConfig(mach=0.5, cfl=1.0, precision=_lib.PREC_FP64, ordering=_lib.ORDER_SPATIAL)
+    state = perturbed_state(arrays, flow, 3)
+    n = int(arrays["n_cells"])
+    scaled = {k: v.copy() for k, v in state.items()}
+    for key in ("rho", "p"):
+        scaled[key][:n] *= 2.0 ** power
+    inner = np.ones(n, bool)  # without the cells of farfield faces, whose ghosts keep the freestream
+    inner[arrays["farfield_interior"]] = False
+    want = residual(arrays, flow, state, kernel)[inner]
+    got = residual(arrays, flow, scaled, kernel)[inner] * 2.0 ** -power
+    assert np.max(np.abs(got - want)) <= 8 * 2e-13 * np.max(np.abs(want))
