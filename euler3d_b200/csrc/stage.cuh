@@ -439,6 +439,26 @@ __device__ __forceinline__ void ghost_store(double *gp, double rho, double u, do
 // single-precision fluxes.
 enum : int { PREC_EXACT = 0, PREC_FAST = 1, PREC_F32 = 2 };
 
+// 1 / c, 1 / (rho c) and rho c of a sound speed from one root: with r = 1 / sqrt(gamma p rho), of the
+// density's sign, they are rho r, r and gamma p rho r.  Where that product is zero, infinite or no number these
+// are not what the reference's quotients are (0 x inf for a pressure of zero, say); the hardware's coarse
+// approximations have the quotients' own zeros, infinities and NaN.  Quotients for those cases cost the
+// FP32_FLUX kernel spills at nine blocks per SM, inlined (16.8 -> 17.5 ms for 40 iterations of 1.57M
+// tetrahedra) or called (17.5).
+__device__ __forceinline__ double3 inverse_sound(double g, double p, double rho) {
+    const double x = g * p * rho, r = copysign(rsqrt_nr(x), rho);
+    double3 s = make_double3(rho * r, r, x * r);
+    if (x == 0.0 || !(fabs(x) < HUGE_VAL)) {
+        double ir, c;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ir) : "d"(rho));
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(s.x) : "d"(g * (p * ir)));
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(c) : "d"(s.x));
+        s.z = rho * c;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(s.y) : "d"(s.z));
+    }
+    return s;
+}
+
 // Tail shared by subsonic farfield, wall and symmetry ghosts (src/solver/PhysicalBC.cpp:62-66); c is the
 // interior cell's sound speed in exact mode and its reciprocal otherwise (two fast reciprocals and a
 // root instead of three divisions and a root).
@@ -454,7 +474,7 @@ __device__ __forceinline__ void ghost_finish(double *gp, double g, double rho, d
     } else {
         const double q2 = fma(u, u, fma(v, v, w * w));
         const double e = p * rcp_nr((g - 1.0) * rho);  // internal energy; p / rho = (gamma - 1) e
-        M = (q2 == 0.0 ? 0.0 : q2 * rsqrt_nr(q2)) * c;
+        M = (q2 > 0.0 && q2 < HUGE_VAL ? q2 * rsqrt_nr(q2) : q2) * c;
         E = fma(0.5, q2, e);
         H = fma(g - 1.0, e, E);
     }
@@ -476,7 +496,7 @@ __device__ __forceinline__ void ghost_mirror(double *gp, double g, const Prim &d
     double v = d.v - 2 * V * ny;
     double w = d.w - 2 * V * nz;
     if (store) {
-        const double c = PREC == PREC_EXACT ? sqrt(g * (d.p / d.rho)) : fabs(d.rho) * rsqrt_nr(g * d.p * d.rho);
+        const double c = PREC == PREC_EXACT ? sqrt(g * (d.p / d.rho)) : inverse_sound(g, d.p, d.rho).x;
         ghost_finish<PREC>(gp, g, d.rho, u, v, w, d.p, c, out);
     } else {
         double H = 0.0;
@@ -531,8 +551,8 @@ __device__ __forceinline__ void ghost_farfield(double *gp, double g, const Frees
         }
         ghost_finish<PREC>(gp, g, rho, u, v, w, p, c, out);
     } else {
-        // with r = 1 / sqrt(gamma p rho), of the density's sign: 1/c = rho r, 1/(rho c) = r, rho c = gamma p rho r
-        const double gpr = g * d.p * d.rho, r = copysign(rsqrt_nr(gpr), d.rho), ic = d.rho * r;
+        const double3 s = inverse_sound(g, d.p, d.rho);
+        const double ic = s.x, r = s.y;
         double p, rho, u, v, w;
         if (V > 0.0) {
             const double dpr = (d.p - fs.p) * r;
@@ -543,7 +563,7 @@ __device__ __forceinline__ void ghost_farfield(double *gp, double g, const Frees
             w = fma(nz, dpr, d.w);
         } else {
             const double dV = fma(nx, fs.u - d.u, fma(ny, fs.v - d.v, nz * (fs.w - d.w)));
-            p = 0.5 * (fs.p + d.p - gpr * r * dV);
+            p = 0.5 * (fs.p + d.p - s.z * dV);
             const double dpr = (p - fs.p) * r;
             rho = fma(p - fs.p, ic * ic, fs.rho);
             u = fma(nx, dpr, fs.u);

@@ -138,3 +138,31 @@ def test_roe_of_densities_out_of_range(power, kernel):
     want = residual(arrays, flow, state, kernel)[inner]
     got = residual(arrays, flow, scaled, kernel)[inner] * 2.0 ** -power
     assert np.max(np.abs(got - want)) <= 8 * 2e-13 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_FP32_FLUX])
+@pytest.mark.parametrize("key,value", [("p", 0.0), ("rho", 0.0), ("p", 1e-30), ("p", np.inf), ("rho", np.inf),
+                                       ("u", np.inf), ("v", -np.inf), ("p", np.nan), ("rho", np.nan), ("w", np.nan)])
+@pytest.mark.parametrize("name", ["channel", "ogrid", "tets"])
+def test_ghosts_of_cells_out_of_range(name, key, value, precision):
+    """Ghosts of cells with a zero, vanishing, infinite or undefined entry, of every boundary kind: NaN and
+    infinite where the exact mode's are, and the same numbers elsewhere (30 roundings, as above)."""
+    arrays = prepared(name)
+    n = int(arrays["n_cells"])
+    state = perturbed_state(arrays, FlowConfig(mach=0.5), 3)
+    state[key][np.flatnonzero(np.random.default_rng(5).uniform(size=n) < 0.3)] = value
+    got = []
+    for prec in (_lib.PREC_FP64_EXACT, precision):
+        flow = FlowConfig(mach=0.5, cfl=1.0, precision=prec, ordering=_lib.ORDER_SPATIAL)
+        s = EulerSolver(arrays, flow, autotune=False)
+        s.set_state(state)
+        s.residual()
+        got.append(s.get_state())
+        s.close()
+    tol = 900 * (2.0 ** -53 if precision == _lib.PREC_FP64 else 2.0 ** -24)
+    for k in ("rho", "u", "v", "w", "p", "E", "H", "M"):
+        want, have = got[0][k][n:], got[1][k][n:]
+        assert np.array_equal(np.isnan(want), np.isnan(have)), k
+        assert np.array_equal(np.isinf(want), np.isinf(have)), k
+        w, h = want[np.isfinite(want)], have[np.isfinite(want)]
+        assert np.max(np.abs(h - w) / (np.abs(w) + np.median(np.abs(w)))) <= tol, k
