@@ -404,8 +404,8 @@ __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double n
         double pp;
         if (fabs(M) <= 1.0) pp = 0.25 * (M + 1.0) * (M + 1.0) * (2.0 - M);
         else pp = M > 0.0 ? 1.0 : 0.0;
-        f = fma(0.0, V, 2.0 * pp * d.p);  // NaN where V is no finite number, as the general flux's products
-        energy = 0.0 * (d.rho * V * d.H);
+        f = fma(0.0, M, 2.0 * pp * d.p);  // NaN where M is no finite number, as the general flux's products
+        energy = 0.0 * (M * d.H);
     } else {
         double qt2 = fma(d.u, d.u, fma(d.v, d.v, d.w * d.w)), h = d.H;
         if (loaded) {
@@ -415,7 +415,8 @@ __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double n
         }
         qt2 = fma(-V, V, qt2);
         const double c2 = (g - 1.0) * fma(-0.5, qt2, h);
-        f = fma(d.rho * V, V + c2 * rsqrt_nr(sign_or(c2, d.rho)), d.p);  // NaN for a negative density
+        // NaN for a negative density or pressure, as the general flux's roots
+        f = fma(d.rho * V, V + c2 * rsqrt_nr(sign_or(sign_or(c2, d.rho), d.p)), d.p);
     }
     F[0] = 0.0;
     F[1] = f * nx;

@@ -166,3 +166,19 @@ def test_ghosts_of_cells_out_of_range(name, key, value, precision):
         assert np.array_equal(np.isinf(want), np.isinf(have)), k
         w, h = want[np.isfinite(want)], have[np.isfinite(want)]
         assert np.max(np.abs(h - w) / (np.abs(w) + np.median(np.abs(w)))) <= tol, k
+
+
+@pytest.mark.parametrize("kernel", DOUBLE_KERNELS)
+@pytest.mark.parametrize("scheme", [_lib.SCHEME_ROE, _lib.SCHEME_AUSM])
+@pytest.mark.parametrize("key", ["p", "rho"])
+def test_symmetry_faces_of_one_negative_entry(key, scheme, kernel):
+    """A negative pressure or density alone has no sound speed: NaN through a symmetry face, as in the
+    exact mode."""
+    arrays = cube()
+    out = []
+    for prec, k in ((_lib.PREC_FP64_EXACT, _lib.KERNEL_TILE), (_lib.PREC_FP64, kernel)):
+        flow = FlowConfig(mach=0.5, cfl=1.0, precision=prec, scheme=scheme)
+        state = perturbed_state(arrays, flow, 3)
+        state[key][0] *= -1.0
+        out.append(residual(arrays, flow, state, k)[0, 1:4])
+    assert np.isnan(out[0]).all() and np.isnan(out[1]).all()
