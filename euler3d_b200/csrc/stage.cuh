@@ -447,7 +447,12 @@ enum : int { PREC_EXACT = 0, PREC_FAST = 1, PREC_F32 = 2 };
 // FP32_FLUX kernel spills at nine blocks per SM, inlined (16.8 -> 17.5 ms for 40 iterations of 1.57M
 // tetrahedra) or called (17.5).
 __device__ __forceinline__ double3 inverse_sound(double g, double p, double rho) {
-    const double x = g * p * rho, r = copysign(rsqrt_nr(x), rho);
+    const double x = g * p * rho;
+    if (seed_ok(__double2hiint(x))) {
+        const double r = copysign(rsqrt_nr(x), rho);
+        return make_double3(rho * r, r, x * r);
+    }
+    const double r = copysign(rsqrt(x), rho);
     double3 s = make_double3(rho * r, r, x * r);
     if (x == 0.0 || !(fabs(x) < HUGE_VAL)) {
         double ir, c;
@@ -475,7 +480,10 @@ __device__ __forceinline__ void ghost_finish(double *gp, double g, double rho, d
     } else {
         const double q2 = fma(u, u, fma(v, v, w * w));
         const double e = p * rcp_nr((g - 1.0) * rho);  // internal energy; p / rho = (gamma - 1) e
-        M = (q2 > 0.0 && q2 < HUGE_VAL ? q2 * rsqrt_nr(q2) : q2) * c;
+        double speed = q2;  // zero, infinite and undefined ones as they are
+        if (seed_ok(__double2hiint(q2))) speed = q2 * rsqrt_nr(q2);
+        else if (q2 > 0.0 && q2 < HUGE_VAL) speed = q2 * rsqrt(q2);
+        M = speed * c;
         E = fma(0.5, q2, e);
         H = fma(g - 1.0, e, E);
     }
