@@ -398,13 +398,15 @@ static __device__ __noinline__ double mirror_enthalpy(double p, double rho, doub
 __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double ny, double nz, double g, int scheme,
                                               bool loaded, double F[5]) {
     const double V = fma(d.u, nx, fma(d.v, ny, d.w * nz));
-    double f, energy = 0.0;
+    double f, mass = 0.0, energy = 0.0;
     if (scheme == 1) {
-        const double M = V * (d.rho * rsqrt_nr(g * d.p * d.rho));
+        const double r = rsqrt_nr(g * d.p * d.rho), M = V * (d.rho * r);
         double pp;
         if (fabs(M) <= 1.0) pp = 0.25 * (M + 1.0) * (M + 1.0) * (2.0 - M);
         else pp = M > 0.0 ? 1.0 : 0.0;
-        f = fma(0.0, M, 2.0 * pp * d.p);  // NaN where M is no finite number, as the general flux's products
+        // NaN where M (for the mass, the sound speed) is no finite number, as the general flux's products
+        f = fma(0.0, M, 2.0 * pp * d.p);
+        mass = 0.0 * r;
         energy = 0.0 * (M * d.H);
     } else {
         double qt2 = fma(d.u, d.u, fma(d.v, d.v, d.w * d.w)), h = d.H;
@@ -417,8 +419,10 @@ __device__ __forceinline__ void sym_flux_fast(const Prim &d, double nx, double n
         const double c2 = (g - 1.0) * fma(-0.5, qt2, h);
         // NaN for a negative density or pressure, as the general flux's roots
         f = fma(d.rho * V, V + c2 * rsqrt_nr(sign_or(sign_or(c2, d.rho), d.p)), d.p);
+        mass = 0.0 * f;
+        energy += mass;
     }
-    F[0] = 0.0;
+    F[0] = mass;
     F[1] = f * nx;
     F[2] = f * ny;
     F[3] = f * nz;
